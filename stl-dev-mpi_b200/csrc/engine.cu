@@ -1170,6 +1170,24 @@ class EngineImpl final : public Engine {
               if (cell >= 0) rows[u].push_back({cell, cmax(&coef[((i64)(8 * c + p) * op.n_rep + u) * 8])});
             }
         }
+      } else if (op.grid) {
+        auto start = fetch(op.g_start, (i64*)nullptr);
+        auto off = fetch(op.g_off, (int32_t*)nullptr);
+        auto pos = fetch(op.g_pos, (int32_t*)nullptr);
+        auto coef = fetch_real(op.g_coef, op.dtype);
+        const int VL = 16 / (int)dsize(op.dtype);
+        auto squeeze = [](int v) { return (v & 1) | ((v >> 1) & 2) | ((v >> 2) & 4); };
+        for (i64 u = 0; u < op.n_rep; ++u) {
+          const i64 tile = u / kGridRows;
+          const int ul = (int)(u % kGridRows);
+          const int p0 = (squeeze(ul >> 1) + kGridHalo) * kGridP + squeeze(ul) + kGridHalo;
+          for (i64 sl = start[tile]; sl < start[tile + 1]; ++sl) {
+            double c[8];
+            for (int j = 0; j < 8; ++j) c[j] = coef[((sl * (8 / VL) + j / VL) * kGridRows + ul) * VL + j % VL];
+            const int32_t cell = pos[tile * kGridCells + p0 + off[sl]];
+            if (cell >= 0 && cmax(c) != 0.0) rows[u].push_back({cell, cmax(c)});
+          }
+        }
       } else {
         auto cell = fetch(op.cell, (int32_t*)nullptr);
         auto coef = fetch_real(op.coef, op.dtype);
@@ -1225,7 +1243,7 @@ class EngineImpl final : public Engine {
     std::vector<std::array<int, 4>> v;
     for (const auto& c : conv_)
       v.push_back({c.mma ? c.m_S : c.S, c.mma ? c.m_pc : c.max_tile_cells,
-                   c.mma_adj ? 3 : c.mma ? 2 : c.colored ? 1 : 0, c.mma_adj ? c.m_wl : 0});
+                   c.mma_adj ? 3 : c.mma ? 2 : c.colored || c.grid ? 1 : 0, c.mma_adj ? c.m_wl : 0});
     return v;
   }
 
@@ -1722,7 +1740,7 @@ class EngineImpl final : public Engine {
       if (cand.size() < 2) return 0;
       std::ostringstream k;
       k << dev << '|' << what << '|' << opt_.fp32 << '|' << R << '|' << B;
-      if (op) k << '|' << op->n_rep << '|' << op->S << '|' << op->nk << '|' << op->colored << '|' << op->max_tile_cells;
+      if (op) k << '|' << op->n_rep << '|' << op->S << '|' << op->nk << '|' << (op->grid ? 2 : (int)op->colored) << '|' << op->max_tile_cells;
       if (dop) k << '|' << dop->n_rep_out << '|' << dop->n_rep_in << '|' << dop->W << '|' << dop->WT << '|' << dop->nk;
       const std::string key = k.str();
       {

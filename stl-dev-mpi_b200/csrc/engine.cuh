@@ -162,6 +162,20 @@ struct ConvOp {
   DevMem tile_off;           // uint16 [n_tiles][nch][ncs]: first entry of (chunk, tile cell)
   DevMem coff;               // int64 [stored cells + 1]
   DevMem clist;              // uint32 tile << 12 | tile cell << 2 | rotation
+  // Grid layout (full sky, nside >= 16): tiles of kGridRows stored rows, an 8 x 8
+  // pixel block of one face.  A slot of a tile is one displacement (dx, dy) of
+  // the face frame, the same for all its rows, so the cells of a slot are the
+  // tile's block moved by it: no index per row, no two rows on one cell, and
+  // regular shared-memory addresses.  The displacements of the rows of a tile
+  // differ little (128 rows at nside 1024: 45.6 of them a tile for 44.4 cells a
+  // row; 64: 53.6 for 44.1; 16: 66.3 for 44.0), so the slots hold no more padding
+  // than a colouring of the tile's entries (48 slots) does.
+  bool grid = false;
+  DevMem g_start;            // int64 [n_tiles + 1]: first slot of every tile (a multiple of kGridPad)
+  DevMem g_off;              // int32 [slots]: dy kGridP + dx
+  DevMem g_coef;             // T [slots][8 / VL][kGridRows][VL], VL values of T in 16 bytes
+  DevMem g_pos;              // int32 [n_tiles][kGridCells]: the cell at every grid position (-1: none)
+  DevMem g_lpos;             // uint16 [n_tiles][ncs]: grid position of every tile cell
   int G = 4;
   double mean_slots = 0.0;   // cells read per row, averaged over the rows
   // Tensor-core layout (FP32 full sky; replaces the coloured one).  Tiles of
@@ -190,7 +204,7 @@ struct ConvOp {
   size_t bytes() const {
     return cell.bytes + coef.bytes + tent.bytes + coefT.bytes + rowsum.bytes + tile_cells.bytes + tile_ncells.bytes +
            tile_slots.bytes + lcell.bytes + lcell_t.bytes + tile_ent.bytes + tile_off.bytes + coff.bytes +
-           clist.bytes + m_coef.bytes + m_cells.bytes + m_lc.bytes + m_wlc.bytes + m_winv.bytes + m_rowch.bytes +
+           clist.bytes + g_start.bytes + g_off.bytes + g_coef.bytes + g_pos.bytes + g_lpos.bytes + m_coef.bytes + m_cells.bytes + m_lc.bytes + m_wlc.bytes + m_winv.bytes + m_rowch.bytes +
            m_tch.bytes;
   }
 };
@@ -204,6 +218,17 @@ __host__ __device__ constexpr int mma_class(int p) { return (0x23013210 >> (4 * 
 constexpr int kAdjTile = 128;    // stored rows per tile of the tiled forward and adjoint
 constexpr int kAdjCells = 1024;  // cells a tile may read
 constexpr int kAdjSC = 8;        // slots per chunk of the two-phase adjoint
+// Grid layout: rows of a tile by local NESTED index, x bits 0 2 4 and y bits
+// 1 3 5; the tile's cells on a grid with a halo of kGridHalo cells (the
+// farthest cell a row reads: 5 at the vertices of three faces, 3 or 4
+// elsewhere).  A warp's 32 rows are an 8 x 4 block; its box of cells has the
+// same halo.  The pitch is 4 mod 8 (and mod 16) cells, so the 8 rows (4 x 2) of a
+// quarter warp read 16-byte cells of distinct banks.
+constexpr int kGridRows = 64, kGridHalo = 5, kGridMin = 16;  // kGridMin: least nside
+constexpr int kGridP = 20, kGridW = 8 + 2 * kGridHalo, kGridCells = kGridP * kGridW;
+constexpr int kBoxH = 4 + 2 * kGridHalo, kBoxCells = kGridP * kBoxH;
+constexpr int kGridPad = 4;  // a tile's slots are padded to a multiple (zero coefficients, no displacement)
+constexpr int kGridSlots = (2 * kGridHalo + 1) * (2 * kGridHalo + 1);  // most displacements of a tile
 
 // Scratch of the row-centric adjoint: the tile partial sums
 // [n_tiles][4][ncs][R] (capacity bytes).

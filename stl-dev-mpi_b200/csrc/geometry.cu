@@ -229,22 +229,22 @@ __global__ void k_conv_coefT(const uint32_t* tent, const T* coef, i64 n_rep, int
   }
 }
 
-// Adjoint tiles: one block per tile of kAdjTile stored rows.  The cells the
+// Adjoint tiles: one block per tile of TR stored rows.  The cells the
 // tile's rows read (all slots) are sorted in shared memory (bitonic), made
 // unique, written to the tile's list, and every (slot, row) gets the index
 // of its cell in that list.
-__global__ void k_adj_tiles(const int32_t* cell, int S, i64 n_rep, int P2, int32_t* tile_cells, int32_t* tile_nc,
+__global__ void k_adj_tiles(const int32_t* cell, int S, i64 n_rep, int TR, int P2, int32_t* tile_cells, int32_t* tile_nc,
                             uint16_t* lcell, int* overflow) {
   extern __shared__ int32_t buf[];  // [P2] sorted cells, then [kAdjCells] unique, then [256] counts
   int32_t* uniq = buf + P2;
   int32_t* cnt = uniq + kAdjCells;
   const int tid = threadIdx.x;
-  const i64 u0 = (i64)blockIdx.x * kAdjTile;
-  const int n = S * kAdjTile;
+  const i64 u0 = (i64)blockIdx.x * TR;
+  const int n = S * TR;
   for (int i = tid; i < P2; i += blockDim.x) {
     int32_t v = 0x7fffffff;
     if (i < n) {
-      const int s = i / kAdjTile, ul = i % kAdjTile;
+      const int s = i / TR, ul = i % TR;
       if (u0 + ul < n_rep) v = cell[(i64)s * n_rep + u0 + ul];
     }
     buf[i] = v;
@@ -286,7 +286,7 @@ __global__ void k_adj_tiles(const int32_t* cell, int S, i64 n_rep, int P2, int32
   __syncthreads();
   const int nc = min(tile_nc[blockIdx.x], kAdjCells);
   for (int i = tid; i < n; i += blockDim.x) {
-    const int s = i / kAdjTile, ul = i % kAdjTile;
+    const int s = i / TR, ul = i % TR;
     if (u0 + ul >= n_rep) continue;
     const int32_t v = cell[(i64)s * n_rep + u0 + ul];
     int lo = 0, hi = nc;
@@ -523,6 +523,103 @@ __global__ void k_color_apply(const int32_t* cell, const T* coef, const uint16_t
     lcell2[e2] = lcell[e];
     for (int j = 0; j < 8; ++j) coef2[e2 * 8 + j] = coef[e * 8 + j];
   }
+}
+
+// Grid layout, one block of kGridRows threads per tile, thread = row.  Pass 0
+// counts the tile's distinct displacements; pass 1 (g_start set, g_coef
+// zeroed) writes the slots in (dy, dx) order, the coefficients, the cell at
+// every grid position and the position of every tile cell.  *fail: a cell
+// beyond the halo, or positions and cells that are not one to one.
+template <typename T>
+struct GridArgs {
+  const int32_t* cell;
+  const int* counts;
+  const T* coef;
+  i64 n_rep, nside;
+  int order;
+  int32_t* nslots;
+  const i64* start;
+  int32_t* off;
+  T* gcoef;
+  int32_t* pos;
+  const int32_t* tile_cells;
+  const int32_t* tile_nc;
+  int ncs;
+  uint16_t* lpos;
+  int* fail;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kGridRows) k_grid_layout(GridArgs<T> a, int pass) {
+  constexpr int D = 2 * kGridHalo + 1, VL = 16 / (int)sizeof(T);
+  __shared__ int present[kGridSlots], rank[kGridSlots];
+  __shared__ int32_t spos[kGridCells];
+  __shared__ int found;
+  const int row = threadIdx.x;
+  const i64 tile = blockIdx.x, u = tile * kGridRows + row;
+  for (int i = row; i < kGridSlots; i += kGridRows) present[i] = 0;
+  for (int i = row; i < kGridCells; i += kGridRows) spos[i] = -1;
+  if (row == 0) found = 0;
+  __syncthreads();
+  const int o2 = 2 * a.order;
+  const i64 pix = ((4 * (u >> o2)) << o2) | (u & ((i64(1) << o2) - 1));  // the stored row's pixel
+  i64 x, y, f;
+  nest2xyf(pix, a.order, x, y, f);
+  const int px = (int)(x & 7), py = (int)(y & 7), cnt = a.counts[u];
+  int bad = 0;
+  for (int s = 0; s < cnt; ++s) {
+    int dx, dy;
+    if (rel_cell(f, x, y, a.cell[(i64)s * a.n_rep + u], a.nside, a.order, kGridHalo, dx, dy))
+      present[(dy + kGridHalo) * D + dx + kGridHalo] = 1;
+    else
+      bad = 1;
+  }
+  if (bad) atomicExch(a.fail, 1);
+  __syncthreads();
+  if (row == 0) {
+    int n = 0;
+    for (int i = 0; i < kGridSlots; ++i) {
+      rank[i] = n;
+      n += present[i];
+    }
+    if (pass == 0) a.nslots[tile] = (n + kGridPad - 1) / kGridPad * kGridPad;
+  }
+  __syncthreads();
+  if (pass == 0 || bad) return;
+  const i64 s0 = a.start[tile];
+  for (int i = row; i < kGridSlots; i += kGridRows)
+    if (present[i]) {
+      const int dy = i / D - kGridHalo, dx = i % D - kGridHalo;
+      a.off[s0 + rank[i]] = dy * kGridP + dx;
+    }
+  for (int s = 0; s < cnt; ++s) {
+    const i64 e = (i64)s * a.n_rep + u;
+    const int32_t c = a.cell[e];
+    int dx, dy;
+    if (!rel_cell(f, x, y, c, a.nside, a.order, kGridHalo, dx, dy)) continue;
+    const i64 slot = s0 + rank[(dy + kGridHalo) * D + dx + kGridHalo];
+    for (int j = 0; j < 8; ++j) a.gcoef[((slot * (8 / VL) + j / VL) * kGridRows + row) * VL + j % VL] = a.coef[e * 8 + j];
+    const int old = atomicCAS(&spos[(py + kGridHalo + dy) * kGridP + px + kGridHalo + dx], -1, c);
+    if (old != -1 && old != c) atomicExch(a.fail, 1);
+  }
+  __syncthreads();
+  const int nc = a.tile_nc[tile];
+  const int32_t* tc = a.tile_cells + tile * kAdjCells;
+  for (int i = row; i < kGridCells; i += kGridRows) {
+    const int32_t c = spos[i];
+    a.pos[tile * kGridCells + i] = c;
+    if (c < 0) continue;
+    int lo = 0, hi = nc;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (tc[mid] < c) lo = mid + 1; else hi = mid;
+    }
+    if (lo < nc && tc[lo] == c) a.lpos[tile * a.ncs + lo] = (uint16_t)i;
+    else atomicExch(a.fail, 1);
+    atomicAdd(&found, 1);
+  }
+  __syncthreads();
+  if (row == 0 && found != nc) atomicExch(a.fail, 1);
 }
 
 // lcell [S][n_rep] -> tile-major [n_tiles][nch * 4][kAdjTile] (slots padded
@@ -1134,6 +1231,62 @@ static bool build_mma_layout(ConvOp& op, const DevMem& counts, bool adjoint, cud
   return true;
 }
 
+// The grid layout of a full-sky operator (ConvOp::g_*) from its per-row slots
+// and tile cells; false (nothing kept) when a tile does not fit it.
+template <typename T>
+static bool build_grid_layout(ConvOp& op, const DevMem& counts, i64 nside, int order, cudaStream_t s) {
+  DevMem nslots(sizeof(int32_t) * op.n_tiles), flag(sizeof(int));
+  STL_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
+  GridArgs<T> a{};
+  a.cell = op.cell.as<int32_t>();
+  a.counts = counts.as<int>();
+  a.coef = op.coef.as<T>();
+  a.n_rep = op.n_rep;
+  a.nside = nside;
+  a.order = order;
+  a.nslots = nslots.as<int32_t>();
+  a.tile_cells = op.tile_cells.as<int32_t>();
+  a.tile_nc = op.tile_ncells.as<int32_t>();
+  a.ncs = op.max_tile_cells + 1;
+  a.fail = flag.as<int>();
+  k_grid_layout<T><<<(unsigned)op.n_tiles, kGridRows, 0, s>>>(a, 0);
+  STL_CUDA(cudaGetLastError());
+  if (read_flag(flag, s)) return false;
+  std::vector<int32_t> n(op.n_tiles);
+  STL_CUDA(cudaMemcpyAsync(n.data(), nslots.p, nslots.bytes, cudaMemcpyDeviceToHost, s));
+  STL_CUDA(cudaStreamSynchronize(s));
+  std::vector<i64> start(op.n_tiles + 1, 0);
+  int most = 1;
+  for (i64 t = 0; t < op.n_tiles; ++t) {
+    start[t + 1] = start[t] + n[t];
+    most = std::max(most, (int)n[t]);
+  }
+  const i64 slots = start[op.n_tiles];
+  DevMem g_start(sizeof(i64) * (op.n_tiles + 1)), g_off(sizeof(int32_t) * std::max<i64>(slots, 1)),
+      g_coef(sizeof(T) * 8 * kGridRows * std::max<i64>(slots, 1)), g_pos(sizeof(int32_t) * kGridCells * op.n_tiles),
+      g_lpos(sizeof(uint16_t) * (size_t)a.ncs * op.n_tiles);
+  STL_CUDA(cudaMemcpyAsync(g_start.p, start.data(), g_start.bytes, cudaMemcpyHostToDevice, s));
+  STL_CUDA(cudaMemsetAsync(g_coef.p, 0, g_coef.bytes, s));
+  STL_CUDA(cudaMemsetAsync(g_off.p, 0, g_off.bytes, s));
+  STL_CUDA(cudaMemsetAsync(g_lpos.p, 0, g_lpos.bytes, s));
+  a.start = g_start.as<i64>();
+  a.off = g_off.as<int32_t>();
+  a.gcoef = g_coef.as<T>();
+  a.pos = g_pos.as<int32_t>();
+  a.lpos = g_lpos.as<uint16_t>();
+  k_grid_layout<T><<<(unsigned)op.n_tiles, kGridRows, 0, s>>>(a, 1);
+  STL_CUDA(cudaGetLastError());
+  if (read_flag(flag, s)) return false;
+  op.g_start = std::move(g_start);
+  op.g_off = std::move(g_off);
+  op.g_coef = std::move(g_coef);
+  op.g_pos = std::move(g_pos);
+  op.g_lpos = std::move(g_lpos);
+  op.S = most;
+  op.ncs = a.ncs;
+  return true;
+}
+
 template <typename T>
 static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, ConvOp& op, cudaStream_t s) {
   const int P = sp.ksz * sp.ksz;
@@ -1179,6 +1332,7 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
   // of kAdjTile stored rows, then the edge colouring of its entries
   op.adj_tiles = false;
   op.colored = false;
+  op.grid = false;
   op.mma = op.mma_adj = false;
   if (std::is_same<T, float>::value && sym && sp.tensor_cores > 0) {
     // FP32 full sky: the tensor-core layout when every tile fits it, for the
@@ -1200,32 +1354,38 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
     }
   }
   if (sym && op.S <= 128) {  // the tile sort holds 128 slots per row
-    op.n_tiles = (a.n_rows + kAdjTile - 1) / kAdjTile;
-    op.tile_slots.alloc(sizeof(int32_t) * op.n_tiles);
-    k_tile_slots<<<nblocks(op.n_tiles, 256), 256, 0, s>>>(counts.as<int>(), a.n_rows, op.n_tiles,
-                                                          op.tile_slots.as<int32_t>());
-    STL_CUDA(cudaGetLastError());
-    op.tile_cells.alloc(sizeof(int32_t) * kAdjCells * op.n_tiles);
-    op.tile_ncells.alloc(sizeof(int32_t) * op.n_tiles);
     op.lcell.alloc(sizeof(uint16_t) * op.S * a.n_rows);
-    int P2 = 1;
-    while (P2 < op.S * kAdjTile) P2 <<= 1;
-    const size_t smem = sizeof(int32_t) * ((size_t)P2 + kAdjCells + 256);
-    if (smem > 48 * 1024)
-      allow_dynamic_smem(k_adj_tiles);
-    STL_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
-    k_adj_tiles<<<(unsigned)op.n_tiles, 256, smem, s>>>(op.cell.as<int32_t>(), op.S, a.n_rows, P2,
-                                                          op.tile_cells.as<int32_t>(), op.tile_ncells.as<int32_t>(),
-                                                          op.lcell.as<uint16_t>(), flag.as<int>());
-    STL_CUDA(cudaGetLastError());
-    op.adj_tiles = !read_flag(flag, s);
-    std::vector<int32_t> nc(op.n_tiles);
-    STL_CUDA(cudaMemcpyAsync(nc.data(), op.tile_ncells.p, sizeof(int32_t) * op.n_tiles, cudaMemcpyDeviceToHost, s));
-    STL_CUDA(cudaStreamSynchronize(s));
-    op.max_tile_cells = 0;
-    for (int32_t v : nc) op.max_tile_cells = std::max(op.max_tile_cells, (int)v);
-    if ((uint64_t)op.n_tiles >= (1ull << 20)) op.adj_tiles = false;
-    if (op.adj_tiles && op.max_tile_cells < kAdjCells) {
+    allow_dynamic_smem(k_adj_tiles);
+    // the distinct cells of every tile of TR stored rows
+    auto make_tiles = [&](int TR) {
+      op.n_tiles = (a.n_rows + TR - 1) / TR;
+      op.tile_cells.alloc(sizeof(int32_t) * kAdjCells * op.n_tiles);
+      op.tile_ncells.alloc(sizeof(int32_t) * op.n_tiles);
+      int P2 = 1;
+      while (P2 < op.S * TR) P2 <<= 1;
+      P2 = std::max(P2, 256);  // an entry per thread of the sort's block
+      const size_t smem = sizeof(int32_t) * ((size_t)P2 + kAdjCells + 256);
+      STL_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
+      k_adj_tiles<<<(unsigned)op.n_tiles, 256, smem, s>>>(op.cell.as<int32_t>(), op.S, a.n_rows, TR, P2,
+                                                            op.tile_cells.as<int32_t>(), op.tile_ncells.as<int32_t>(),
+                                                            op.lcell.as<uint16_t>(), flag.as<int>());
+      STL_CUDA(cudaGetLastError());
+      op.adj_tiles = !read_flag(flag, s);
+      op.max_tile_cells = device_max(op.tile_ncells.as<int32_t>(), op.n_tiles, s);
+      if ((uint64_t)op.n_tiles >= (1ull << 20)) op.adj_tiles = false;
+    };
+    if (sp.nside >= kGridMin && !op.mma) {
+      make_tiles(kGridRows);
+      op.grid = op.adj_tiles && op.max_tile_cells <= kGridCells && build_grid_layout<T>(op, counts, sp.nside, a.order, s);
+    }
+    if (!op.grid) {
+      make_tiles(kAdjTile);
+      op.tile_slots.alloc(sizeof(int32_t) * op.n_tiles);
+      k_tile_slots<<<nblocks(op.n_tiles, 256), 256, 0, s>>>(counts.as<int>(), a.n_rows, op.n_tiles,
+                                                            op.tile_slots.as<int32_t>());
+      STL_CUDA(cudaGetLastError());
+    }
+    if (!op.grid && op.adj_tiles && op.max_tile_cells < kAdjCells) {
       // every colour a matching: the coloured layout replaces the slots
       DevMem col((size_t)op.S * a.n_rows), tile_d(sizeof(int32_t) * op.n_tiles);
       const size_t csm = color_smem(op.S);
@@ -1256,10 +1416,17 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
   }
   if (!op.rowsum.p) {  // the row sums (the tensor-core branch made them already)
     op.rowsum.alloc(sizeof(T) * 8 * a.n_rows);
-    k_rowsum<T><<<nblocks(a.n_rows, 256), 256, 0, s>>>(op.coef.as<T>(), op.S, a.n_rows, op.rowsum.as<T>());
+    const int slots = op.grid ? (int)(op.coef.bytes / (sizeof(T) * 8 * a.n_rows)) : op.S;
+    k_rowsum<T><<<nblocks(a.n_rows, 256), 256, 0, s>>>(op.coef.as<T>(), slots, a.n_rows, op.rowsum.as<T>());
     STL_CUDA(cudaGetLastError());
   }
-  if (!op.colored) {
+  if (op.grid) {  // its own coefficients replace the per-row slots
+    STL_CUDA(cudaStreamSynchronize(s));
+    op.cell.release();
+    op.coef.release();
+    op.lcell.release();
+  }
+  if (!op.colored && !op.grid) {
     // transposed gather table over the stored cells: entries (u, s, j)
     int sbits = 1;
     while ((1 << sbits) < op.S) ++sbits;
@@ -1287,7 +1454,7 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
   if (!op.adj_tiles) return;
   op.nch = (op.S + kAdjSC - 1) / kAdjSC;
   op.ncs = op.max_tile_cells + 1;
-  if (!op.colored) {
+  if (!op.colored && !op.grid) {
     // per tile and slot chunk: the entries of every tile cell
     op.tile_ent.alloc(sizeof(uint16_t) * (size_t)op.n_tiles * op.S * kAdjTile);
     op.tile_off.alloc(sizeof(uint16_t) * (size_t)op.n_tiles * op.nch * op.ncs);
@@ -1303,7 +1470,7 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
       STL_CUDA(cudaGetLastError());
     }
   }
-  {
+  if (!op.grid) {
     const int S4 = ((op.S + 3) / 4) * 4;
     op.lcell_t.alloc(sizeof(uint16_t) * (size_t)op.n_tiles * S4 * kAdjTile);
     const i64 n = op.n_tiles * S4 * kAdjTile;
@@ -1338,6 +1505,7 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
     k_adj_csort<<<nblocks(n_in_rep, 256), 256, 0, s>>>(op.coff.as<i64>(), n_in_rep, op.clist.as<uint32_t>());
     STL_CUDA(cudaGetLastError());
     STL_CUDA(cudaStreamSynchronize(s));
+    if (op.grid) op.tile_cells.release();  // its kernels find the cells by grid position
   }
   STL_CUDA(cudaStreamSynchronize(s));
 }

@@ -313,4 +313,34 @@ HD bool ext_pix(i64 face, i64 ex, i64 ey, i64 nside, int order, i64& out) {
   return true;
 }
 
+// offsets (dx, dy), each at most `reach`, whose extended coordinates around
+// pixel (x, y) of `face` are the cell (the inverse of ext_pix near a pixel);
+// false when the cell is not that near
+HD bool rel_cell(i64 face, i64 x, i64 y, i64 cell, i64 nside, int order, int reach, int& dx, int& dy) {
+  const signed char NB_FACE[9][12] = {
+      {8, 9, 10, 11, -1, -1, -1, -1, 10, 11, 8, 9}, {5, 6, 7, 4, 8, 9, 10, 11, 9, 10, 11, 8},
+      {-1, -1, -1, -1, 5, 6, 7, 4, -1, -1, -1, -1}, {4, 5, 6, 7, 11, 8, 9, 10, 11, 8, 9, 10},
+      {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11},       {1, 2, 3, 0, 0, 1, 2, 3, 5, 6, 7, 4},
+      {-1, -1, -1, -1, 7, 4, 5, 6, -1, -1, -1, -1}, {3, 0, 1, 2, 3, 0, 1, 2, 4, 5, 6, 7},
+      {2, 3, 0, 1, -1, -1, -1, -1, 0, 1, 2, 3}};
+  const unsigned char NB_SWAP[9][3] = {{0, 0, 3}, {0, 0, 6}, {0, 0, 0}, {0, 0, 5}, {0, 0, 0},
+                                       {5, 0, 0}, {0, 0, 0}, {6, 0, 0}, {3, 0, 0}};
+  i64 cx, cy, cf;
+  nest2xyf(cell, order, cx, cy, cf);
+  for (int nb = 0; nb < 9; ++nb) {
+    if (NB_FACE[nb][face] != cf) continue;
+    i64 a = cx, b = cy;
+    const int bits = NB_SWAP[nb][face >> 2];
+    if (bits & 4) { i64 t = a; a = b; b = t; }
+    if (bits & 2) b = nside - b - 1;
+    if (bits & 1) a = nside - a - 1;
+    const i64 ex = a + (nb % 3 - 1) * nside - x, ey = b + (nb / 3 - 1) * nside - y;
+    if (ex < -reach || ex > reach || ey < -reach || ey > reach) continue;
+    dx = (int)ex;
+    dy = (int)ey;
+    return true;
+  }
+  return false;
+}
+
 }  // namespace stl

@@ -885,6 +885,542 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
   }
 }
 
+// ---- grid wavelets (ConvOp::grid) ----------------------------------------------
+// A thread takes one stored row, all its 4 rotations and RB field rows; lanes
+// are consecutive rows (an 8 x 4 pixel block a warp).  Per slot a thread loads
+// its 8 coefficients once for 4 RB field values, so FP32 at RB = 4 makes 128
+// FMAs from 2 coefficient and 4 cell loads of 16 bytes: 24 shared-memory
+// wavefronts per 4096 FMAs of a warp (the per-slot gathers of k_conv_fwd_tiles
+// take 37), every one of them full: the 8 rows of a quarter warp read distinct
+// banks, the coefficients lying in planes of 16 bytes a row and the cells at the
+// grid's pitch.  A CTA holds FG groups of RB rows over one tile, which share its
+// coefficients: they arrive once a CTA by bulk copies, in stages of grid_sc()
+// slots.  Measured on one B200 (nside 1024, J 9, B 4, FP32, a forward and its
+// VJP): forward 14.5 -> 9.6 ms, adjoint 21.4 -> 15.5 ms; FP64, nside 512, J 8, B 1: 2.80 ->
+// 2.03 and 5.02 -> 2.73 ms.  The level-0 branch forward at nside 512 keeps the FMA
+// pipe 57 % busy (36 % before) with three CTAs an SM of 168 registers a thread; two
+// CTAs (no spills, 255 registers) took 11 % longer.  What bounds it now is the FMA
+// pipe inside the slot loop (about 170 of 160 cycles a slot and scheduler) and
+// the CTAs' prologues and epilogues (a third of their time, partly hidden).
+template <typename T>
+__host__ __device__ constexpr int grid_vl() { return 16 / (int)sizeof(T); }  // values of 16 bytes
+template <typename T>
+__host__ __device__ constexpr int grid_sc() { return sizeof(T) == 4 ? 4 : 2; }  // slots of a stage (8 KB)
+constexpr int kGridStages = 3;
+constexpr int kGridSlot = kGridRows * 8;  // values of a slot
+constexpr size_t kGridStageBytes = 8192;
+
+// x and y (3 bits each) of a row of a tile, local NESTED index
+__device__ __forceinline__ int grid_x(int ul) { return (ul & 1) | ((ul >> 1) & 2) | ((ul >> 2) & 4); }
+__device__ __forceinline__ int grid_y(int ul) { return grid_x(ul >> 1); }
+
+// The coefficient stream of a CTA: stage c % kGridStages holds the slots
+// c SC .. of the tile.  Thread 0 fills a stage by one bulk copy; every warp
+// waits for it on its own and releases it with one arrival; a stage is
+// refilled a chunk after it was released, so the refill seldom waits.  Every
+// wait is bounded.
+template <typename T, int WARPS>
+struct GridStream {
+  static constexpr int SC = grid_sc<T>();
+  static_assert(SC * kGridSlot * sizeof(T) == kGridStageBytes && kGridPad % SC == 0, "whole stages");
+  unsigned char* base;
+  uint64_t *full, *empty;
+  const T* src;  // the tile's first coefficient
+  int S, nch, issued;
+  __device__ __forceinline__ void init() {  // thread 0
+    for (int q = 0; q < kGridStages; ++q) {
+      mbar_init(&full[q], 1);
+      mbar_init(&empty[q], WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __device__ __forceinline__ void issue(int c) {  // thread 0
+    const int st = c % kGridStages;
+    mbar_expect_tx(&full[st], kGridStageBytes);
+    bulk_g2s(base + st * kGridStageBytes, src + (i64)c * SC * kGridSlot, kGridStageBytes, &full[st]);
+    issued = c + 1;
+  }
+  __device__ __forceinline__ bool wait(int c) { return mbar_wait(&full[c % kGridStages], (c / kGridStages) & 1); }
+  __device__ __forceinline__ const T* stage(int c) const {
+    return reinterpret_cast<const T*>(base + (c % kGridStages) * kGridStageBytes);
+  }
+  // after chunk c was read by the warp; thread 0 refills the stage of chunk c - 1
+  __device__ __forceinline__ bool release(int c, int tid) {
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&empty[c % kGridStages]);
+    if (tid == 0 && c > 0 && c - 1 + kGridStages < nch) {
+      if (!mbar_wait(&empty[(c - 1) % kGridStages], ((c - 1) / kGridStages) & 1)) return false;
+      issue(c - 1 + kGridStages);
+    }
+    return true;
+  }
+  // thread 0, after a failed wait anywhere: the copies in flight land (bounded)
+  __device__ __forceinline__ int drain() {
+    bool ok = true;
+    for (int q = max(0, issued - kGridStages); q < issued; ++q) ok &= wait(q);
+    return ok ? kErrWait : kErrDrain;
+  }
+};
+
+// The RB field rows of a thread.  FP32 pairs of rows sit in 64-bit registers and
+// share the paired FMA (each component rounded as fmaf, so results do not
+// depend on RB).
+template <typename T, int RB> struct GridRows {  // FP64, or one FP32 row
+  T v[RB];
+};
+template <> struct GridRows<float, 2> { uint64_t v[1]; };
+template <> struct GridRows<float, 4> { uint64_t v[2]; };
+// a coefficient as the factor of a pair
+template <typename T, int RB> struct GridCoef { T w; };
+template <> struct GridCoef<float, 2> { uint64_t w; };
+template <> struct GridCoef<float, 4> { uint64_t w; };
+
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+template <typename T, int RB>
+__device__ __forceinline__ GridCoef<T, RB> gr_coef(T w) {
+  GridCoef<T, RB> c;
+  if constexpr (sizeof(T) == 4 && RB > 1)
+    asm volatile("mov.b64 %0, {%1, %1};" : "=l"(c.w) : "f"(w));  // once a slot
+  else
+    c.w = w;
+  return c;
+}
+template <typename T, int RB>
+__device__ __forceinline__ GridRows<T, RB> gr_pack(const T (&x)[RB]) {
+  GridRows<T, RB> a;
+  if constexpr (sizeof(T) == 4 && RB > 1) {
+#pragma unroll
+    for (int i = 0; i < RB / 2; ++i) a.v[i] = pack2(x[2 * i], x[2 * i + 1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < RB; ++i) a.v[i] = x[i];
+  }
+  return a;
+}
+template <typename T, int RB>
+__device__ __forceinline__ T gr_at(const GridRows<T, RB>& a, int i) {
+  if constexpr (sizeof(T) == 4 && RB > 1) {
+    const float2 p = unpack2(a.v[i >> 1]);
+    return i & 1 ? p.y : p.x;
+  } else {
+    return a.v[i];
+  }
+}
+// a + w b, w b, a + b
+template <typename T, int RB>
+__device__ __forceinline__ void gr_fma(GridRows<T, RB>& a, const GridCoef<T, RB>& w, const GridRows<T, RB>& b) {
+  if constexpr (sizeof(T) == 4 && RB > 1) {
+#pragma unroll
+    for (int i = 0; i < RB / 2; ++i) a.v[i] = fma2(w.w, b.v[i], a.v[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < RB; ++i) a.v[i] = fma(w.w, b.v[i], a.v[i]);
+  }
+}
+template <typename T, int RB>
+__device__ __forceinline__ GridRows<T, RB> gr_mul(const GridCoef<T, RB>& w, const GridRows<T, RB>& b) {
+  GridRows<T, RB> a;
+  if constexpr (sizeof(T) == 4 && RB > 1) {
+#pragma unroll
+    for (int i = 0; i < RB / 2; ++i) a.v[i] = mul2(w.w, b.v[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < RB; ++i) a.v[i] = w.w * b.v[i];
+  }
+  return a;
+}
+template <typename T, int RB>
+__device__ __forceinline__ void gr_add(GridRows<T, RB>& a, const GridRows<T, RB>& b) {
+  if constexpr (sizeof(T) == 4 && RB > 1) {
+#pragma unroll
+    for (int i = 0; i < RB / 2; ++i) a.v[i] = add2(a.v[i], b.v[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < RB; ++i) a.v[i] += b.v[i];
+  }
+}
+// RB values at an address aligned to them (shared or global memory), one access
+template <typename T, int RB> struct GridVec;
+template <> struct GridVec<float, 1> { typedef float type; };
+template <> struct GridVec<float, 2> { typedef unsigned long long type; };
+template <> struct GridVec<float, 4> { typedef ulonglong2 type; };
+template <> struct GridVec<double, 1> { typedef double type; };
+template <> struct GridVec<double, 2> { typedef double2 type; };
+template <typename T, int RB>
+__device__ __forceinline__ GridRows<T, RB> gr_load(const T* p) {
+  const typename GridVec<T, RB>::type q = *reinterpret_cast<const typename GridVec<T, RB>::type*>(p);
+  GridRows<T, RB> a;
+  static_assert(sizeof(q) == sizeof(a), "one vector");
+  memcpy(&a, &q, sizeof(a));
+  return a;
+}
+template <typename T, int RB>
+__device__ __forceinline__ void gr_store(T* p, const GridRows<T, RB>& a) {
+  typename GridVec<T, RB>::type q;
+  memcpy(&q, &a, sizeof(a));
+  *reinterpret_cast<typename GridVec<T, RB>::type*>(p) = q;
+}
+// the 8 coefficients of a staged slot (planes of 16 bytes a row)
+__device__ __forceinline__ void grid_coef(const float* p, float (&w)[8]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float4 a = *reinterpret_cast<const float4*>(p + q * kGridRows * 4);
+    w[4 * q] = a.x; w[4 * q + 1] = a.y; w[4 * q + 2] = a.z; w[4 * q + 3] = a.w;
+  }
+}
+__device__ __forceinline__ void grid_coef(const double* p, double (&w)[8]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double2 a = *reinterpret_cast<const double2*>(p + q * kGridRows * 2);
+    w[2 * q] = a.x; w[2 * q + 1] = a.y;
+  }
+}
+// The complex outputs (cotangents) of a CTA, 4 rotations x kGridRows pixels,
+// pieces of FG RB x 8 values contiguous in the field: they pass through shared
+// memory (pieces 16 bytes apart, so a thread's 16-byte accesses fall in
+// distinct banks) and consecutive threads move consecutive 16 bytes of them.  A
+// thread's own vector accesses of the field touch 32 lines an instruction (a
+// third of the L1 wavefronts of the two kernels), and one bulk copy a piece
+// takes about 25 cycles of the copy engine each: 6 400 cycles for a CTA's 256.
+template <typename T, int RB, int FG>
+__host__ __device__ constexpr int grid_piece() { return FG * RB * 8 * (int)sizeof(T); }
+template <typename T, int RB, int FG>
+__host__ __device__ constexpr size_t grid_pieces_bytes() { return (size_t)4 * kGridRows * (grid_piece<T, RB, FG>() + 16); }
+
+// threads an SM holds: 384 of 168 registers (FP32 at RB = 4, FP64 at RB = 2), else 640
+template <typename T, int RB, int FG>
+__host__ __device__ constexpr int grid_fwd_ctas() { return (RB * (int)sizeof(T) == 16 ? 384 : 640) / (kGridRows * FG); }
+
+template <typename T, int RB, int FG>
+__global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) k_conv_fwd_grid(
+    const T* __restrict__ coef, const i64* __restrict__ start, const int32_t* __restrict__ off,
+    const int32_t* __restrict__ pos, int o2, const T* __restrict__ x, int R, T* __restrict__ out,
+    const T* __restrict__ rowsum, const double* __restrict__ rc, int* __restrict__ err) {
+  constexpr int SC = grid_sc<T>(), NT = kGridRows * FG, VL = grid_vl<T>();
+  constexpr int kPlanes = 4 * kGridCells * RB;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(16) int soff[kGridSlots + 7];
+  __shared__ __align__(8) uint64_t bar[2 * kGridStages];
+  __shared__ int fail;
+  T* planes = reinterpret_cast<T*>(smem_raw + kGridStages * kGridStageBytes);  // [FG][4][kGridCells][RB]
+  const int ngroups = R / (RB * FG);  // CTAs of a tile: consecutive, so its coefficients stay in L2
+  const i64 tile = blockIdx.x / ngroups;
+  const int tid = threadIdx.x, row = tid % kGridRows, fg = tid / kGridRows;
+  const int rg = (int)(blockIdx.x % ngroups) * RB * FG, r0 = rg + fg * RB;
+  // loads that depend on nothing, before the first wait
+  constexpr int NP = (kGridCells * FG + NT - 1) / NT;
+  int32_t cell[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int q = tid + i * NT;
+    cell[i] = q < kGridCells * FG ? __ldg(pos + tile * kGridCells + q / FG) : -1;
+  }
+  const i64 u = tile * kGridRows + row;
+  T rs[8];
+  load8(rowsum + u * 8, rs);
+  const i64 s0 = start[tile];
+  GridStream<T, NT / 32> cs;
+  cs.base = smem_raw;
+  cs.full = bar;
+  cs.empty = bar + kGridStages;
+  cs.src = coef + s0 * kGridSlot;
+  cs.S = (int)(start[tile + 1] - s0);
+  cs.nch = cs.S / SC;  // a tile's slots are whole stages
+  cs.issued = 0;
+  // the tile's cells, 4 rotations x RB rows a group; positions no row reads: zero
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int q = tid + i * NT;
+    if (q >= kGridCells * FG) break;
+    const int32_t c = cell[i];
+    T* dst = planes + (size_t)(q % FG) * kPlanes + (q / FG) * RB;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      cp_async_r<RB * sizeof(T)>(dst + (size_t)k * kGridCells * RB,
+                                 x + (c >= 0 ? rot_cell(c, k, o2) * R + rg + (q % FG) * RB : 0), c >= 0);
+  }
+  if (tid == 0) {
+    cs.init();
+    fail = 0;
+    for (int c = 0; c < min(cs.nch, kGridStages); ++c) cs.issue(c);
+  }
+  for (int i = tid; i < cs.S; i += NT) soff[i] = off[s0 + i] * RB;
+  // the sums start from the rows' constants times the row sums of the coefficients
+  GridRows<T, RB> acc[4][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    T v[RB];
+#pragma unroll
+    for (int rb = 0; rb < RB; ++rb) v[rb] = rc ? (T)(rc[r0 + rb] * (double)rs[j]) : (T)0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k][j] = gr_pack<T, RB>(v);
+  }
+  const T* px = planes + (size_t)fg * kPlanes + ((grid_y(row) + kGridHalo) * kGridP + grid_x(row) + kGridHalo) * RB;
+  cp_async_wait_all();
+  __syncthreads();
+  bool ok = true;
+  for (int c = 0; c < cs.nch; ++c) {
+    if (!cs.wait(c)) {
+      ok = false;
+      break;
+    }
+    const T* cf = cs.stage(c) + row * VL;
+#pragma unroll
+    for (int sl = 0; sl < SC; ++sl) {
+      asm volatile("" ::: "memory");  // one slot's loads at a time: four slots' would spill
+      T w[8];
+      grid_coef(cf + sl * kGridSlot, w);
+      const T* p = px + soff[c * SC + sl];
+      GridRows<T, RB> xv[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) xv[k] = gr_load<T, RB>(p + (size_t)k * kGridCells * RB);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const GridCoef<T, RB> wj = gr_coef<T, RB>(w[j]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) gr_fma(acc[k][j], wj, xv[k]);
+      }
+    }
+    if (!cs.release(c, tid)) {
+      ok = false;
+      break;
+    }
+  }
+  if (!ok) fail = 1;
+  __syncthreads();
+  if (fail) {
+    if (tid == 0) atomicMax(err, cs.drain());
+    return;
+  }
+  // every stage has landed and been read: the outputs take the shared memory
+  constexpr int PB = grid_piece<T, RB, FG>(), PS = PB + 16;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    T* dst = reinterpret_cast<T*>(smem_raw + (size_t)(k * kGridRows + row) * PS) + fg * RB * 8;
+#pragma unroll
+    for (int rb = 0; rb < RB; ++rb) {
+      T o[8];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        o[2 * g] = gr_at(acc[k][2 * rot_src(k, g)], rb);
+        const T im = gr_at(acc[k][2 * rot_src(k, g) + 1], rb);
+        o[2 * g + 1] = rot_conj(k, g) ? -im : im;
+      }
+      store8(dst + rb * 8, o);
+    }
+  }
+  __syncthreads();
+  constexpr int PC = PB / 16;  // 16-byte units of a piece: consecutive threads write consecutive ones
+#pragma unroll 1
+  for (int k = 0; k < 4; ++k) {
+    unsigned char* ob = reinterpret_cast<unsigned char*>(out + (rot_pixel(tile * kGridRows, k, o2) * R + rg) * 8);
+    const unsigned char* sb = smem_raw + (size_t)k * kGridRows * PS;
+#pragma unroll
+    for (int i = 0; i < kGridRows * PC / NT; ++i) {
+      const int q = (tid + i * NT) / PC, c = (tid + i * NT) % PC;
+      *reinterpret_cast<uint4*>(ob + (size_t)q * R * (8 * sizeof(T)) + c * 16) =
+          *reinterpret_cast<const uint4*>(sb + q * PS + c * 16);
+    }
+  }
+}
+
+// Adjoint: the same threads; the row's cotangents under the 4 rotations stay in
+// registers, and per slot a thread adds its 4 RB products into its cell's sums
+// in its warp's own box of shared memory: the rows of a warp reach distinct
+// cells in a slot, and no other warp touches the box, so the slots need
+// __syncwarp only (the coloured adjoint's barrier per slot, shared by 16 warps,
+// was its largest stall).  Every cell sums its products in slot order, then
+// the warps' boxes are added in warp order into the tile's partials: results
+// are bit-reproducible.  40 wavefronts per 4096 FMAs of a warp (the coloured
+// kernel: 59).
+template <typename T, int RB, int FG>
+__host__ __device__ constexpr int grid_adj_ctas() { return (RB * (int)sizeof(T) == 16 ? 256 : 384) / (kGridRows * FG); }
+
+template <typename T, int RB, int FG>
+__global__ void __launch_bounds__(kGridRows * FG, (grid_adj_ctas<T, RB, FG>())) k_conv_adj_grid(
+    const T* __restrict__ coef, const i64* __restrict__ start, const int32_t* __restrict__ off,
+    const uint16_t* __restrict__ lpos, const int32_t* __restrict__ tile_nc, int ncs, int o2,
+    const T* __restrict__ gy, int R, T* __restrict__ part, ModulusAdd<T> madd, int* __restrict__ err) {
+  constexpr int SC = grid_sc<T>(), NT = kGridRows * FG, VL = grid_vl<T>();
+  constexpr int kBox = 4 * kBoxCells * RB;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(16) int soff[kGridSlots + 7];
+  __shared__ __align__(8) uint64_t bar[2 * kGridStages];
+  __shared__ int fail;
+  constexpr int PB = grid_piece<T, RB, FG>(), PS = PB + 16;
+  unsigned char* pieces = smem_raw + kGridStages * kGridStageBytes;  // the cotangents, then the boxes
+  T* boxes = reinterpret_cast<T*>(smem_raw + kGridStages * kGridStageBytes);  // [warps][4][kBoxCells][RB]
+  const int ngroups = R / (RB * FG);
+  const i64 tile = blockIdx.x / ngroups;
+  const int tid = threadIdx.x, row = tid % kGridRows, fg = tid / kGridRows, lane = tid & 31;
+  const int rg = (int)(blockIdx.x % ngroups) * RB * FG, r0 = rg + fg * RB;
+  constexpr int PC = PB / 16;  // the cotangents, 16 bytes a copy, consecutive threads on consecutive ones
+#pragma unroll 1
+  for (int k = 0; k < 4; ++k) {
+    const unsigned char* gb = reinterpret_cast<const unsigned char*>(gy + (rot_pixel(tile * kGridRows, k, o2) * R + rg) * 8);
+    unsigned char* pb = pieces + (size_t)k * kGridRows * PS;
+#pragma unroll
+    for (int i = 0; i < kGridRows * PC / NT; ++i) {
+      const int q = (tid + i * NT) / PC, c = (tid + i * NT) % PC;
+      cp_async16(pb + q * PS + c * 16, gb + (size_t)q * R * (8 * sizeof(T)) + c * 16, 16);
+    }
+  }
+  const i64 s0 = start[tile];
+  GridStream<T, NT / 32> cs;
+  cs.base = smem_raw;
+  cs.full = bar;
+  cs.empty = bar + kGridStages;
+  cs.src = coef + s0 * kGridSlot;
+  cs.S = (int)(start[tile + 1] - s0);
+  cs.nch = cs.S / SC;  // a tile's slots are whole stages
+  cs.issued = 0;
+  if (tid == 0) {
+    cs.init();
+    fail = 0;
+    for (int c = 0; c < min(cs.nch, kGridStages); ++c) cs.issue(c);
+  }
+  for (int i = tid; i < cs.S; i += NT) soff[i] = off[s0 + i] * RB;
+  // the combine's positions of this thread's tile cells
+  const int nc = tile_nc[tile];
+  constexpr int NL = (kGridCells * FG + NT - 1) / NT;
+  int ps[NL];
+#pragma unroll
+  for (int i = 0; i < NL; ++i) {
+    const int j = tid + i * NT;
+    ps[i] = j < nc * FG ? (int)lpos[tile * ncs + j / FG] : 0;
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  GridRows<T, RB> g[4][8];
+  const i64 u = tile * kGridRows + row;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const i64 p = rot_pixel(u, k, o2);
+    T t[8][RB];  // by stored (gauge, re/im): the gauge permutation and conjugation folded in
+#pragma unroll
+    for (int rb = 0; rb < RB; ++rb) {
+      T c[8];
+      load8_shared(reinterpret_cast<const T*>(pieces + (size_t)(k * kGridRows + row) * PS) + (fg * RB + rb) * 8, c);
+      if (madd.z) {  // the modulus VJP of row r0 + rb (map b): c += g z / |z|
+        T zz[8];
+        load8(madd.z + (p * R + r0 + rb) * 8, zz);
+        const T* gm = madd.g + p * madd.g_pix + (i64)(r0 + rb) * madd.g_row;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const T mag = zabs(zz[2 * l], zz[2 * l + 1]);
+          const T dd = mag == (T)0 ? (T)1 : mag;
+          const T gv = gm[l];
+          c[2 * l] += gv * zz[2 * l] / dd;
+          c[2 * l + 1] += gv * zz[2 * l + 1] / dd;
+        }
+      }
+#pragma unroll
+      for (int gg = 0; gg < 4; ++gg) {
+        const int q = rot_src(k, gg);
+        t[2 * q][rb] = c[2 * gg];
+        t[2 * q + 1][rb] = rot_conj(k, gg) ? -c[2 * gg + 1] : c[2 * gg + 1];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) g[k][q] = gr_pack<T, RB>(t[q]);
+  }
+  __syncthreads();  // every thread has its cotangents (and the displacements are in): the boxes
+  T* box = boxes + (tid >> 5) * kBox;
+  for (int i = lane; i < kBox / VL; i += 32) reinterpret_cast<uint4*>(box)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  T* sum = box + ((grid_y(lane) + kGridHalo) * kGridP + grid_x(lane) + kGridHalo) * RB;
+  bool ok = true;
+  for (int c = 0; c < cs.nch; ++c) {
+    if (!cs.wait(c)) {
+      ok = false;
+      break;
+    }
+    const T* cf = cs.stage(c) + row * VL;
+    T w[8];
+    grid_coef(cf, w);
+#pragma unroll
+    for (int sl = 0; sl < SC; ++sl) {
+      T* p = sum + soff[c * SC + sl];
+      GridRows<T, RB> v[4], a[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = gr_load<T, RB>(p + (size_t)k * kBoxCells * RB);
+      T wn[8];  // the next slot's coefficients, ahead of this slot's stores
+      if (sl + 1 < SC) grid_coef(cf + (sl + 1) * kGridSlot, wn);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const GridCoef<T, RB> wq = gr_coef<T, RB>(w[q]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (q == 0) a[k] = gr_mul(wq, g[k][0]);
+          else gr_fma(a[k], wq, g[k][q]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        gr_add(v[k], a[k]);
+        gr_store(p + (size_t)k * kBoxCells * RB, v[k]);
+      }
+      __syncwarp();  // the slot's sums are in: another row of the warp may read them
+      if (sl + 1 < SC)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) w[q] = wn[q];
+    }
+    if (!cs.release(c, tid)) {
+      ok = false;
+      break;
+    }
+  }
+  if (!ok) fail = 1;
+  __syncthreads();
+  if (fail) {
+    if (tid == 0) atomicMax(err, cs.drain());
+    return;
+  }
+  // partials [tile][k][ncs][R]: a cell's sums of the two warps (upper and lower
+  // 8 x 4 block) of each group
+#pragma unroll
+  for (int i = 0; i < NL; ++i) {  // consecutive threads: the groups of one cell, then cells
+    const int j = tid + i * NT;
+    if (j >= nc * FG) break;
+    const int lc = j / FG, f = j % FG;
+    const T* b = boxes + (size_t)(2 * f) * kBox + (size_t)ps[i] * RB;
+    const bool lower = ps[i] < kBoxH * kGridP, upper = ps[i] >= 4 * kGridP;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      GridRows<T, RB> a{};
+      if (lower) a = gr_load<T, RB>(b + (size_t)k * kBoxCells * RB);
+      if (upper) gr_add(a, gr_load<T, RB>(b + kBox + (size_t)k * kBoxCells * RB - 4 * kGridP * RB));
+      gr_store(part + ((tile * 4 + k) * ncs + lc) * R + rg + f * RB, a);
+    }
+  }
+}
+
 // gx[rotation k' of stored cell v][r] (+)= sum over the entries (tile, lc, j)
 // of v, in order, of part[tile][(k' - j) mod 4][lc][r]
 template <typename T, int NK, int RB>
@@ -2231,6 +2767,44 @@ size_t adjc_smem(const ConvOp& op) {
          sizeof(T) * (size_t)op.ncs * 4 * RB;
 }
 
+template <typename T, int RB, int FG>
+void conv_forward_grid_fg(const ConvOp& op, const T* x, int R, T* out, const double* rc, cudaStream_t s, int* err) {
+  const size_t smem = std::max(kGridStages * kGridStageBytes + (size_t)FG * 4 * kGridCells * RB * sizeof(T),
+                               grid_pieces_bytes<T, RB, FG>());
+  allow_dynamic_smem(k_conv_fwd_grid<T, RB, FG>);
+  k_conv_fwd_grid<T, RB, FG><<<(unsigned)(op.n_tiles * (R / (RB * FG))), kGridRows * FG, smem, s>>>(
+      op.g_coef.as<T>(), op.g_start.as<i64>(), op.g_off.as<int32_t>(), op.g_pos.as<int32_t>(), op.o2, x, R, out,
+      op.rowsum.as<T>(), rc, err);
+}
+// two groups of rows a CTA when the rows allow: they share a coefficient stream
+template <typename T, int RB>
+void conv_forward_grid_rb(const ConvOp& op, const T* x, int R, T* out, const double* rc, cudaStream_t s, int* err) {
+  if (R % (2 * RB) == 0) conv_forward_grid_fg<T, RB, 2>(op, x, R, out, rc, s, err);
+  else conv_forward_grid_fg<T, RB, 1>(op, x, R, out, rc, s, err);
+}
+
+template <typename T, int RB, int FG>
+void conv_adjoint_grid_fg(const ConvOp& op, const T* gy, int R, const AdjScratch& scr, cudaStream_t s,
+                          const ModulusAdd<T>* madd, int* err) {
+  const size_t smem = kGridStages * kGridStageBytes +
+                      std::max((size_t)FG * (kGridRows / 32) * 4 * kBoxCells * RB * sizeof(T),
+                               grid_pieces_bytes<T, RB, FG>());
+  allow_dynamic_smem(k_conv_adj_grid<T, RB, FG>);
+  k_conv_adj_grid<T, RB, FG><<<(unsigned)(op.n_tiles * (R / (RB * FG))), kGridRows * FG, smem, s>>>(
+      op.g_coef.as<T>(), op.g_start.as<i64>(), op.g_off.as<int32_t>(), op.g_lpos.as<uint16_t>(),
+      op.tile_ncells.as<int32_t>(), op.ncs, op.o2, gy, R, static_cast<T*>(scr.part), madd ? *madd : ModulusAdd<T>(),
+      err);
+  STL_CUDA(cudaGetLastError());
+}
+template <typename T, int RB>
+void conv_adjoint_grid_rb(const ConvOp& op, const T* gy, int R, T* gx, bool accumulate, const AdjScratch& scr,
+                          cudaStream_t s, const ModulusAdd<T>* madd, int* err) {
+  if (!err) throw std::runtime_error("the grid adjoint needs an error flag");
+  if (R % (2 * RB) == 0) conv_adjoint_grid_fg<T, RB, 2>(op, gy, R, scr, s, madd, err);
+  else conv_adjoint_grid_fg<T, RB, 1>(op, gy, R, scr, s, madd, err);
+  adj_combine_rb<T, RB>(op, R, gx, accumulate, scr, s);
+}
+
 template <typename T, int RB>
 void conv_adjoint_tiles_rb(const ConvOp& op, const T* gy, int R, T* gx, bool accumulate, const AdjScratch& scr,
                            cudaStream_t s, int* err, const ModulusAdd<T>* madd) {
@@ -2419,7 +2993,12 @@ void conv_forward(const ConvOp& op, const T* x, int R, T* out, T* mod, int mod_p
   if (ok.empty() || (rb && std::find(ok.begin(), ok.end(), rb) == ok.end()))
     throw std::runtime_error("invalid wavelet tile height");
   if (!rb) rb = ok.back();  // default: the tallest tile
-  if (forward_tiles(op, sizeof(T), err != nullptr)) {
+  if (op.grid) {
+    if (mod || !err) throw std::runtime_error("the grid wavelet writes no moduli and needs an error flag");
+    if (rb == 4) conv_forward_grid_rb<T, sizeof(T) == 4 ? 4 : 2>(op, x, R, out, rc, s, err);
+    else if (rb == 2) conv_forward_grid_rb<T, 2>(op, x, R, out, rc, s, err);
+    else conv_forward_grid_rb<T, 1>(op, x, R, out, rc, s, err);
+  } else if (forward_tiles(op, sizeof(T), err != nullptr)) {
     if (rb == 4) conv_forward_tiles_rb<T, sizeof(T) == 4 ? 4 : 2>(op, x, R, out, mod, mod_pix, mod_row, mod_off, err,
                                                                   rc, s);
     else if (rb == 2) conv_forward_tiles_rb<T, 2>(op, x, R, out, mod, mod_pix, mod_row, mod_off, err, rc, s);
@@ -2452,7 +3031,9 @@ std::vector<int> conv_forward_choices(const ConvOp& op, size_t elem, int R, bool
   const bool tiles = forward_tiles(op, elem, err);
   for (int rb : {1, 2, 4}) {
     if (R % rb) continue;
-    if (tiles) {
+    if (op.grid) {
+      if (rb * elem > 16) continue;  // a cell's rows are one 16-byte access at most
+    } else if (tiles) {
       if (rb == 4 && elem != 4) continue;
       const size_t sm = elem == 4 ? (rb == 4 ? fwd_tiles_smem<float, 4>(op) : rb == 2 ? fwd_tiles_smem<float, 2>(op)
                                                                                         : fwd_tiles_smem<float, 1>(op))
@@ -2477,6 +3058,7 @@ bool adjoint_tiles_usable(const ConvOp& op, size_t elem, int R, const AdjScratch
     return scr && elem == 4 && adjoint_part_bytes(op, elem, R) <= scr->capacity && adj_mma_smem(op) <= 227 * 1024;
   if (!scr || !op.adj_tiles || op.nk != 4) return false;
   if (adjoint_part_bytes(op, elem, R) > scr->capacity) return false;
+  if (op.grid) return true;
   if (op.colored) return (elem == 4 ? adjc_smem<float, 4>(op) : adjc_smem<double, 1>(op)) <= 227 * 1024;
   const size_t smem = elem == 4 ? (adj_rb(op, elem, R) == 2 ? adj_tiles_smem<float, 2>(op) : adj_tiles_smem<float, 1>(op))
                                 : adj_tiles_smem<double, 1>(op);
@@ -2484,7 +3066,7 @@ bool adjoint_tiles_usable(const ConvOp& op, size_t elem, int R, const AdjScratch
 }
 
 bool conv_adjoint_fuses_modulus(const ConvOp& op, size_t elem, int R, const AdjScratch* scr, int* err) {
-  return (op.colored || op.mma_adj) && err && adjoint_tiles_usable(op, elem, R, scr);
+  return (op.colored || op.grid || op.mma_adj) && err && adjoint_tiles_usable(op, elem, R, scr);
 }
 
 template <typename T>
@@ -2504,7 +3086,14 @@ void conv_adjoint(const ConvOp& op, const T* gy, int R, T* gx, bool accumulate, 
     STL_CUDA(cudaGetLastError());
     return;
   }
-  if (adjoint_tiles_usable(op, sizeof(T), R, scr)) {
+  if (op.grid) {
+    if (!adjoint_tiles_usable(op, sizeof(T), R, scr))
+      throw std::runtime_error("the grid adjoint needs scratch for its tile partials");
+    if (!rb) rb = conv_adjoint_choices(op, sizeof(T), R, scr).back();
+    if (rb == 4) conv_adjoint_grid_rb<T, sizeof(T) == 4 ? 4 : 2>(op, gy, R, gx, accumulate, *scr, s, madd, err);
+    else if (rb == 2) conv_adjoint_grid_rb<T, 2>(op, gy, R, gx, accumulate, *scr, s, madd, err);
+    else conv_adjoint_grid_rb<T, 1>(op, gy, R, gx, accumulate, *scr, s, madd, err);
+  } else if (adjoint_tiles_usable(op, sizeof(T), R, scr)) {
     if (!rb) rb = adj_rb(op, sizeof(T), R);
     if (rb == 4) conv_adjoint_tiles_rb<T, sizeof(T) == 4 ? 4 : 1>(op, gy, R, gx, accumulate, *scr, s, err, madd);
     else if (rb == 2) conv_adjoint_tiles_rb<T, sizeof(T) == 4 ? 2 : 1>(op, gy, R, gx, accumulate, *scr, s, err, madd);
@@ -2535,7 +3124,9 @@ std::vector<int> conv_adjoint_choices(const ConvOp& op, size_t elem, int R, cons
   const bool tiles = adjoint_tiles_usable(op, elem, R, scr);
   for (int rb : {1, 2, 4}) {
     if (R % rb) continue;
-    if (tiles) {
+    if (op.grid) {
+      if (rb * elem > 16) continue;
+    } else if (tiles) {
       if (elem != 4 && rb > 1) continue;
       if (!op.colored && rb == 4) continue;
       if (op.colored && elem == 4 &&

@@ -1,0 +1,39 @@
+"""The full-sky wavelets in the grid layout (levels of nside 16 and more): the
+statistics and their gradient against the FP64 oracle where the layout can go
+wrong -- nside 16, every tile of which reaches across face edges and vertices
+(displacements of 5 cells), the first FP32 level above nside 32, and batches whose
+row counts give a CTA one or two groups of 1, 2 or 4 rows."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nside,J,batch,dtype", [
+    (16, 1, 1, "float64"), (16, 2, 3, "float64"), (32, 2, 2, "float64"),
+    (64, 1, 1, "float32"), (64, 2, 2, "float32"), (64, 1, 3, "float32"), (64, 2, 4, "float32"), (64, 1, 8, "float32")])
+def test_grid_wavelets_match_the_oracle(nside, J, batch, dtype):
+    import stl_b200
+    rng = np.random.default_rng(1000 * nside + 10 * batch + J)
+    x = np.exp(rng.standard_normal((batch, 12 * nside * nside)) - 0.5)
+    e = stl_b200.NativeEngine(nside, J, batch=batch, dtype=dtype)
+    o = O.OracleEngine(nside, J, batch=batch)
+    v, r = e.forward(x)[0], o.forward(x)
+    # FP64: sums of 44 products in another order; FP32: the 1e-6 criterion of the
+    # statistics relative to the largest of their family, and for a gradient
+    # value two chains of at most 44 and 8 rounded products: 52 * 2^-24 = 3.1e-6 of
+    # its largest terms
+    family = np.array([c["family"] for c in e.plan])
+    for f in np.unique(family):
+        a, b = v[:, family == f], r[:, family == f]
+        assert np.max(np.abs(a - b)) <= (1e-12 if dtype == "float64" else 1e-6) * np.max(np.abs(b)), f
+    cot = rng.standard_normal(v.shape) + 1j * rng.standard_normal(v.shape)
+    g, gr = e.vjp(cot), o.vjp(cot)
+    assert np.max(np.abs(g - gr)) <= (1e-11 if dtype == "float64" else 3.1e-6) * np.max(np.abs(gr))
+    again = stl_b200.NativeEngine(nside, J, batch=batch, dtype=dtype, autotune=False)
+    np.testing.assert_array_equal(again.forward(x)[0], v)  # whatever the tile heights
+    np.testing.assert_array_equal(again.vjp(cot), g)
+    e.close()
+    again.close()
