@@ -2387,14 +2387,33 @@ void products0_launch(const ProductShape& sh, const T* z, const T* br, const T* 
   STL_CUDA(cudaGetLastError());
 }
 
-// sums[row][slot] = sum over blocks of partials[blk][row][slot] in block order
-__global__ void k_reduce_partials(const double* __restrict__ partials, int nblk, int rows, int slots,
-                                  double* __restrict__ sums) {
+// sums[row][slot] = sum over blocks of partials[blk][row][slot]: eight threads
+// an output take contiguous runs of blocks, each in block order, added in run
+// order.  One thread an output left 148 to 296 dependent rounds of loads to a few
+// CTAs (31 us at level 0 of nside 512, J 8, B 4; 57 us for the cross sums).
+constexpr int kReduceRuns = 8;
+__global__ void __launch_bounds__(256) k_reduce_partials(const double* __restrict__ partials, int nblk, int rows,
+                                                         int slots, double* __restrict__ sums) {
+  __shared__ double red[kReduceRuns][32];
   const i64 total = (i64)rows * slots;
-  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (i64)gridDim.x * blockDim.x) {
+  const int x = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int k0 = (int)((i64)nblk * r / kReduceRuns), k1 = (int)((i64)nblk * (r + 1) / kReduceRuns);
+  for (i64 i0 = (i64)blockIdx.x * 32; i0 < total; i0 += (i64)gridDim.x * 32) {
+    const i64 i = i0 + x;
     double a = 0.0;
-    for (int k = 0; k < nblk; ++k) a += partials[(i64)k * total + i];
-    sums[i] = a;
+    if (i < total) {
+#pragma unroll 8
+      for (int k = k0; k < k1; ++k) a += partials[(i64)k * total + i];
+    }
+    red[r][x] = a;
+    __syncthreads();
+    if (r == 0 && i < total) {
+      double s = red[0][x];
+#pragma unroll
+      for (int q = 1; q < kReduceRuns; ++q) s += red[q][x];
+      sums[i] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -3282,7 +3301,8 @@ void reduce_partials(const ProductShape& sh, const double* partials, double* sum
     k_reduce_segments<<<grid, 256, 0, s>>>(partials, sh.d_seg_blk, sh.nseg, sh.B * sh.L, sh.slots, sums,
                                            sh.seg_stride);
   } else {
-    k_reduce_partials<<<gx, 256, 0, s>>>(partials, sh.blocks, sh.B * sh.L, sh.slots, sums);
+    k_reduce_partials<<<(unsigned)std::min<i64>((total + 31) / 32, 4096), 256, 0, s>>>(partials, sh.blocks, sh.B * sh.L,
+                                                                                      sh.slots, sums);
   }
   STL_CUDA(cudaGetLastError());
 }
@@ -3759,15 +3779,16 @@ __global__ void __launch_bounds__(kCrossThreads) k_cross_rev(i64 N, int K, int B
   }
 }
 
-// ---- the forward with the four gauges in one CTA (levels with K <= kCross4MaxK) ---
+// ---- the forward with the four gauges in one CTA (K = 13) ---
 // The operands of a (pixel, map, operand) are the 4 gauges' complex values in
 // one run (32 bytes in FP32): a CTA that takes all four gauges of a pixel range
 // loads whole sectors, where one CTA a gauge used a quarter of each (the
 // products of the nside 1024 bench: 17.5 -> 14.3 ms; the same form of the VJP
 // was slower, 22.4 -> 27.2 ms, and is not used).  Staged values
 // sv[j][g][c][i] (i < K the operands, i = K the S1 factor), FP64.
-// levels 0-2 (K = 5, 9, 13): the deeper levels have too few pixel ranges to
-// fill the GPU with a quarter of the CTAs (measured slower at K = 17, 21)
+// level 2 (K = 13; levels 0 and 1 run in registers): the deeper levels have too
+// few pixel ranges to fill the GPU with a quarter of the CTAs (measured slower at
+// K = 17, 21)
 constexpr int kCross4MaxK = 13;
 
 template <typename T>
@@ -3892,6 +3913,230 @@ __global__ void __launch_bounds__(kCrossThreads) k_cross_fwd4(i64 N, int K, int 
   }
 }
 
+// ---- the cross products of the finest levels in registers (K = 5, 9; VJP also 13) ----
+// Levels 0 and 1 hold three quarters of the products.  A thread takes one
+// (pixel, gauge) of a channel pair, gauge fastest, so the four lanes of a
+// (pixel, operand) read its 32-byte run whole, and keeps operands and sums in
+// registers: no staging, no barrier in the loop, and 4 FP64 FMAs of the K^2 per
+// value loaded instead of 4 for two 16-byte shared-memory reads.  The next pixel's operands are
+// loaded while this pixel's products run.
+// Forward: a warp takes RG rows of G (group w % (K / RG) of warp w) and every
+// (warps / groups)-th step of 8 pixels of the CTA's range; lanes, then warps are
+// added in a fixed order into k_cross_fwd's partials.
+// Measured on one B200 (nside 512, J 8, one pair, FP32 fields): forward products of
+// all levels 3.67 -> 1.16 ms (with the shorter ranges of cross_blocks), VJP 3.10 ->
+// 1.36 ms.
+constexpr int kCrossRegThreads = 192;  // 6 warps: 6 streams of K = 5, 2 of 3 row groups at K = 9
+
+template <typename T>
+__device__ __forceinline__ double2 widen(typename V2<T>::type v) {
+  return make_double2((double)v.x, (double)v.y);
+}
+
+template <typename T, bool MOM, int K, int RG>
+__global__ void __launch_bounds__(kCrossRegThreads, MOM ? 1 : 2) k_cross_fwd_reg(
+    i64 N, int Bm, const T* __restrict__ z, const T* __restrict__ br, const uint8_t* __restrict__ mask, i64 chunk,
+    double* __restrict__ partials) {
+  typedef typename V2<T>::type T2;
+  static_assert(K % RG == 0, "whole row groups");
+  constexpr int NG = K / RG, W = kCrossRegThreads / 32, ST = W / NG, K1 = K - 1, L = 4, NV = MOM ? 3 : 2;
+  constexpr int NE = RG * K + 1;  // entries of a thread, the S1 term last
+  extern __shared__ __align__(16) double crs[];  // [W][L][NE][NV]
+  const int B = Bm / 2, b = (int)(blockIdx.x % (unsigned)B);
+  const i64 range = blockIdx.x / (unsigned)B;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l3 = lane & 3, px = lane >> 2;
+  const int grp = warp % NG, stream = warp / NG, row0 = grp * RG;
+  const T2* zv = reinterpret_cast<const T2*>(z);
+  const T2* bv = reinterpret_cast<const T2*>(br);
+  const i64 P0 = range * chunk, P1 = min(N, P0 + chunk);
+  double acc[NE][NV];
+#pragma unroll
+  for (int e = 0; e < NE; ++e)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[e][k] = 0.0;
+  // operand i of channel c: branches, then z (row groups hold rows row0 ..)
+  auto operand = [&](i64 p, int c, int i) {
+    const i64 m = p * Bm + 2 * b + c;
+    return i < K1 ? __ldg(bv + (m * K1 + i) * L + l3) : __ldg(zv + m * L + l3);
+  };
+  T2 a[RG], q[K];
+  bool live = false;
+  auto fetch = [&](i64 p) {
+    live = p < P1 && (!mask || mask[p]);
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < RG; ++i) a[i] = operand(p, 0, row0 + i);
+#pragma unroll
+    for (int i = 0; i < K; ++i) q[i] = operand(p, 1, i);
+  };
+  const i64 step = 8 * ST;
+  fetch(P0 + stream * 8 + px);
+  for (i64 p = P0 + stream * 8; p < P1; p += step) {
+    const bool on = live;
+    T2 ac[RG], qc[K];
+#pragma unroll
+    for (int i = 0; i < RG; ++i) ac[i] = a[i];
+#pragma unroll
+    for (int i = 0; i < K; ++i) qc[i] = q[i];
+    T2 z0c;
+    if (on && grp == 0 && NG > 1) z0c = __ldg(zv + ((p + px) * Bm + 2 * b) * L + l3);
+    fetch(p + step + px);
+    if (!on) continue;
+    double2 v1[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) v1[i] = widen<T>(qc[i]);
+#pragma unroll
+    for (int i = 0; i < RG; ++i) {
+      const double2 v0 = widen<T>(ac[i]);
+      const double n0 = MOM ? fma(v0.x, v0.x, v0.y * v0.y) : 0.0;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        double* s = acc[i * K + k];
+        s[0] = fma(v0.y, v1[k].y, fma(v0.x, v1[k].x, s[0]));
+        s[1] = fma(-v0.x, v1[k].y, fma(v0.y, v1[k].x, s[1]));
+        if (MOM) s[NV - 1] = fma(n0, fma(v1[k].x, v1[k].x, v1[k].y * v1[k].y), s[NV - 1]);
+      }
+    }
+    if (grp == 0) {  // the cross S1: rn(z_0) conj(rn(z_1))
+      const double2 r0 = root_normalise(widen<T>(NG > 1 ? z0c : ac[RG - 1])), r1 = root_normalise(v1[K1]);
+      double* s = acc[NE - 1];
+      s[0] = fma(r0.y, r1.y, fma(r0.x, r1.x, s[0]));
+      s[1] = fma(-r0.x, r1.y, fma(r0.y, r1.x, s[1]));
+      if (MOM) s[NV - 1] = fma(fma(r0.x, r0.x, r0.y * r0.y), fma(r1.x, r1.x, r1.y * r1.y), s[NV - 1]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < NE; ++e)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      double v = acc[e][k];
+      for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (px == 0) crs[(((size_t)warp * L + l3) * NE + e) * NV + k] = v;
+    }
+  __syncthreads();
+  // the streams of a row group in order
+  for (int t = threadIdx.x; t < NG * L * NE; t += kCrossRegThreads) {
+    const int g = t / (L * NE), l = t / NE % L, e = t % NE;
+    if (e == NE - 1 && g > 0) continue;  // the S1 term is group 0's
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int s = 0; s < ST; ++s)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[k] = __dadd_rn(v[k], crs[(((size_t)(s * NG + g) * L + l) * NE + e) * NV + k]);
+    double* out = partials + ((range * B + b) * 4 + l) * cross_slots(K);
+    const int ge = g * RG * K + e;
+    const int at = e < NE - 1 ? 2 * ge : 2 * K * K;
+    out[at] = v[0];
+    out[at + 1] = v[1];
+    out[e < NE - 1 ? 2 * K * K + 2 + ge : 3 * K * K + 2] = v[2];
+  }
+}
+
+// VJP: gv_0 = M v_1 and gv_1 = M^H v_0, plus the cross S1's through rn, as
+// k_cross_rev (the sums over k in the same order).  M of the four gauges in
+// shared memory, FP64.
+constexpr int kCrossRevRegThreads = 128;
+
+template <typename T, int K>
+__global__ void __launch_bounds__(kCrossRevRegThreads, K <= 9 ? 3 : 2) k_cross_rev_reg(
+    i64 N, int Bm, const T* __restrict__ z, const T* __restrict__ br, const T* __restrict__ M, const T* __restrict__ s1,
+    const uint8_t* __restrict__ mask, int accumulate, T* __restrict__ gz, T* __restrict__ gbr) {
+  typedef typename V2<T>::type T2;
+  constexpr int K1 = K - 1, L = 4;
+  __shared__ __align__(16) double2 sm[L * K * K];
+  const int b = blockIdx.y, l3 = threadIdx.x & 3;
+  const T2* Mb = reinterpret_cast<const T2*>(M) + (i64)b * L * K * K;
+  for (int i = threadIdx.x; i < L * K * K; i += kCrossRevRegThreads) sm[i] = widen<T>(Mb[i]);
+  __syncthreads();
+  const double2* mk = sm + l3 * K * K;
+  const double2 sc = widen<T>(reinterpret_cast<const T2*>(s1)[(i64)b * L + l3]);
+  const T2* zv = reinterpret_cast<const T2*>(z);
+  const T2* bv = reinterpret_cast<const T2*>(br);
+  T2* gzv = reinterpret_cast<T2*>(gz);
+  T2* gbv = reinterpret_cast<T2*>(gbr);
+  for (i64 p = (i64)blockIdx.x * (kCrossRevRegThreads / 4) + (threadIdx.x >> 2); p < N;
+       p += (i64)gridDim.x * (kCrossRevRegThreads / 4)) {
+    const bool on = !mask || mask[p];
+    if (!on && accumulate) continue;
+    const i64 m0 = p * Bm + 2 * b, m1 = m0 + 1;
+    T2 a[K], c[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      a[i].x = a[i].y = c[i].x = c[i].y = (T)0;
+      if (on) {
+        a[i] = i < K1 ? __ldg(bv + (m0 * K1 + i) * L + l3) : __ldg(zv + m0 * L + l3);
+        c[i] = i < K1 ? __ldg(bv + (m1 * K1 + i) * L + l3) : __ldg(zv + m1 * L + l3);
+      }
+    }
+    double2 v1[K], g1[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      v1[k] = widen<T>(c[k]);
+      g1[k] = make_double2(0.0, 0.0);
+    }
+    double2 e0 = make_double2(0.0, 0.0), e1 = make_double2(0.0, 0.0);  // the S1 term's
+    if (on) {
+      const double2 z0 = widen<T>(a[K1]), z1 = v1[K1];
+      const double2 r0 = root_normalise(z0), r1 = root_normalise(z1);
+      e0 = root_modulus_vjp(z0, make_double2(__dsub_rn(__dmul_rn(sc.x, r1.x), __dmul_rn(sc.y, r1.y)),
+                                             __dadd_rn(__dmul_rn(sc.x, r1.y), __dmul_rn(sc.y, r1.x))));
+      e1 = root_modulus_vjp(z1, make_double2(__dsub_rn(__dmul_rn(sc.x, r0.x), __dmul_rn(-sc.y, r0.y)),
+                                             __dadd_rn(__dmul_rn(sc.x, r0.y), __dmul_rn(-sc.y, r0.x))));
+    }
+    auto put = [&](T2* dst, double2 g) {
+      T2 o;
+      o.x = (T)g.x;
+      o.y = (T)g.y;
+      if (accumulate) {
+        const T2 prev = *dst;
+        o.x += prev.x;
+        o.y += prev.y;
+      }
+      *dst = o;
+    };
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const double2 v0 = widen<T>(a[i]);
+      double2 g0 = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double2 m = mk[i * K + k];
+        g0.x = fma(m.x, v1[k].x, fma(-m.y, v1[k].y, g0.x));
+        g0.y = fma(m.x, v1[k].y, fma(m.y, v1[k].x, g0.y));
+        g1[k].x = fma(m.x, v0.x, fma(m.y, v0.y, g1[k].x));
+        g1[k].y = fma(m.x, v0.y, fma(-m.y, v0.x, g1[k].y));
+      }
+      if (i == K1) {
+        g0.x += e0.x;
+        g0.y += e0.y;
+        put(gzv + m0 * L + l3, g0);
+      } else {
+        put(gbv + (m0 * K1 + i) * L + l3, g0);
+      }
+    }
+    g1[K1].x += e1.x;
+    g1[K1].y += e1.y;
+#pragma unroll
+    for (int i = 0; i < K; ++i) put(i < K1 ? gbv + (m1 * K1 + i) * L + l3 : gzv + m1 * L + l3, g1[i]);
+  }
+}
+
+template <typename T, bool MOM, int K, int RG>
+void launch_cross_fwd_reg(int nblk, i64 N, int Bm, const T* z, const T* br, const uint8_t* mask, double* partials,
+                          cudaStream_t s) {
+  const size_t smem = sizeof(double) * (kCrossRegThreads / 32) * 4 * (RG * K + 1) * (MOM ? 3 : 2);
+  if (smem > 48 * 1024) allow_dynamic_smem(k_cross_fwd_reg<T, MOM, K, RG>);
+  k_cross_fwd_reg<T, MOM, K, RG><<<(unsigned)nblk * (unsigned)(Bm / 2), kCrossRegThreads, smem, s>>>(
+      N, Bm, z, br, mask, (N + nblk - 1) / nblk, partials);
+}
+
+template <typename T, int K>
+void launch_cross_rev_reg(i64 N, int Bm, const T* z, const T* br, const T* M, const T* s1, const uint8_t* mask,
+                          bool accumulate, T* gz, T* gbr, cudaStream_t s) {
+  const i64 tiles = (N + kCrossRevRegThreads / 4 - 1) / (kCrossRevRegThreads / 4);
+  dim3 grid((unsigned)std::min<i64>(tiles, 148 * 12), (unsigned)(Bm / 2));
+  k_cross_rev_reg<T, K><<<grid, kCrossRevRegThreads, 0, s>>>(N, Bm, z, br, M, s1, mask, accumulate ? 1 : 0, gz, gbr);
+}
+
 template <typename T, bool MOM, int NENT>
 void launch_cross_fwd(unsigned grid, size_t smem, cudaStream_t s, i64 N, int K, int Bm, const T* z, const T* br,
                       const uint8_t* mask, i64 chunk, int PC, double* partials) {
@@ -3926,6 +4171,21 @@ void launch_cross_fwd4(int nent, unsigned grid, size_t smem, cudaStream_t s, i64
 template <typename T>
 void cross_forward(int K, i64 N, int Bm, const T* z, const T* br, const uint8_t* mask, bool moments,
                    double* partials, int nblk, double* sums, cudaStream_t s) {
+  if (K <= 9) {  // in registers
+    if (K == 5) {
+      if (moments) launch_cross_fwd_reg<T, true, 5, 5>(nblk, N, Bm, z, br, mask, partials, s);
+      else launch_cross_fwd_reg<T, false, 5, 5>(nblk, N, Bm, z, br, mask, partials, s);
+    } else {
+      if (moments) launch_cross_fwd_reg<T, true, 9, 3>(nblk, N, Bm, z, br, mask, partials, s);
+      else launch_cross_fwd_reg<T, false, 9, 3>(nblk, N, Bm, z, br, mask, partials, s);
+    }
+    STL_CUDA(cudaGetLastError());
+    const i64 rows = (i64)Bm / 2 * 4, total = rows * cross_slots(K);
+    k_reduce_partials<<<(unsigned)std::min<i64>((total + 31) / 32, 4096), 256, 0, s>>>(partials, nblk, (int)rows,
+                                                                                          cross_slots(K), sums);
+    STL_CUDA(cudaGetLastError());
+    return;
+  }
   if (K <= kCross4MaxK) {  // the four gauges a CTA
     const int E4 = 4 * (K * K + 1), NE = std::min(E4, kCrossThreads), Q = kCrossThreads / NE;
     const int nent = (E4 + NE - 1) / NE;
@@ -3940,7 +4200,7 @@ void cross_forward(int K, i64 N, int Bm, const T* z, const T* br, const uint8_t*
       launch_cross_fwd4<T, false>(nent, grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
     STL_CUDA(cudaGetLastError());
     const i64 rows = (i64)Bm / 2 * 4, total = rows * cross_slots(K);
-    k_reduce_partials<<<(unsigned)std::min<i64>((total + 255) / 256, 1024), 256, 0, s>>>(partials, nblk, (int)rows,
+    k_reduce_partials<<<(unsigned)std::min<i64>((total + 31) / 32, 4096), 256, 0, s>>>(partials, nblk, (int)rows,
                                                                                           cross_slots(K), sums);
     STL_CUDA(cudaGetLastError());
     return;
@@ -3960,7 +4220,7 @@ void cross_forward(int K, i64 N, int Bm, const T* z, const T* br, const uint8_t*
     launch_cross_fwd<T, false>(nent, grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
   STL_CUDA(cudaGetLastError());
   const i64 rows = (i64)Bm / 2 * 4, total = rows * cross_slots(K);
-  k_reduce_partials<<<(unsigned)std::min<i64>((total + 255) / 256, 1024), 256, 0, s>>>(partials, nblk, (int)rows,
+  k_reduce_partials<<<(unsigned)std::min<i64>((total + 31) / 32, 4096), 256, 0, s>>>(partials, nblk, (int)rows,
                                                                                         cross_slots(K), sums);
   STL_CUDA(cudaGetLastError());
 }
@@ -3969,6 +4229,13 @@ template <typename T>
 void cross_reverse(int K, i64 N, int Bm, const T* z, const T* br, const T* M, const T* s1, const uint8_t* mask,
                    bool accumulate, T* gz, T* gbr, cudaStream_t s) {
   if (K > kCrossThreads) throw std::runtime_error("too many operands for the cross VJP");
+  if (K <= 13) {  // in registers
+    if (K == 5) launch_cross_rev_reg<T, 5>(N, Bm, z, br, M, s1, mask, accumulate, gz, gbr, s);
+    else if (K == 9) launch_cross_rev_reg<T, 9>(N, Bm, z, br, M, s1, mask, accumulate, gz, gbr, s);
+    else launch_cross_rev_reg<T, 13>(N, Bm, z, br, M, s1, mask, accumulate, gz, gbr, s);
+    STL_CUDA(cudaGetLastError());
+    return;
+  }
   const int PC = cross_chunk(K);
   const size_t smem = sizeof(double2) * ((size_t)K * K + (size_t)PC * 2 * (K + 1));
   if (smem > 48 * 1024) allow_dynamic_smem(k_cross_rev<T>);
@@ -3981,7 +4248,9 @@ void cross_reverse(int K, i64 N, int Bm, const T* z, const T* br, const T* M, co
   STL_CUDA(cudaGetLastError());
 }
 
-int cross_blocks(i64 N) { return (int)std::max<i64>(1, std::min<i64>(296, (N + 1023) / 1024)); }
+// pixel ranges of the cross sums: 2 an SM, of 64 pixels at least (ranges of 1024
+// gave the levels of nside 64 and less 48 CTAs or fewer: 110-360 us each)
+int cross_blocks(i64 N) { return (int)std::max<i64>(1, std::min<i64>(296, (N + 63) / 64)); }
 
 int means_blocks(i64 N) { return (int)std::max<i64>(1, std::min<i64>(kMeansBlocks, (N + 1023) / 1024)); }
 
