@@ -1875,19 +1875,31 @@ __global__ void k_ell(const int32_t* __restrict__ col, const Tw* __restrict__ w,
   for (int k = 0; k < NK; ++k)
 #pragma unroll
     for (int rb = 0; rb < RB; ++rb) acc[k][rb] = (Tw)0;
-#pragma unroll 4
-  for (int e = 0; e < W; ++e) {  // unrolled: the loads of several entries in flight
-    const i64 idx = (i64)e * n_rep + u;
-    const Tw we = __ldg(w + idx);
-    const i64 c = __ldg(col + idx);
+  // EB entries at a time: their weights and columns, then their values, all in
+  // flight (the sums stay in entry order; past the last entry a zero weight on
+  // the last entry's column)
+  constexpr int EB = NK == 4 && RB <= 2 ? 7 : 4;
+  for (int e0 = 0; e0 < W; e0 += EB) {
+    Tw we[EB];
+    i64 c[EB];
 #pragma unroll
-    for (int k = 0; k < NK; ++k) {
-      const i64 ck = NK == 1 ? c : rot_cell(c, k, o2_in);
-      Tin xv[RB];
-      loadR<RB>(x + ck * x_pix + (i64)ro * x_outer + ri, xv);
-#pragma unroll
-      for (int rb = 0; rb < RB; ++rb) acc[k][rb] = fma(we, (Tw)xv[rb], acc[k][rb]);
+    for (int j = 0; j < EB; ++j) {
+      const i64 idx = (i64)min(e0 + j, W - 1) * n_rep + u;
+      we[j] = e0 + j < W ? __ldg(w + idx) : (Tw)0;
+      c[j] = __ldg(col + idx);
     }
+    Tin xv[EB][NK][RB];
+#pragma unroll
+    for (int j = 0; j < EB; ++j)
+#pragma unroll
+      for (int k = 0; k < NK; ++k)
+        loadR<RB>(x + (NK == 1 ? c[j] : rot_cell(c[j], k, o2_in)) * x_pix + (i64)ro * x_outer + ri, xv[j][k]);
+#pragma unroll
+    for (int j = 0; j < EB; ++j)
+#pragma unroll
+      for (int k = 0; k < NK; ++k)
+#pragma unroll
+        for (int rb = 0; rb < RB; ++rb) acc[k][rb] = fma(we[j], (Tw)xv[j][k][rb], acc[k][rb]);
   }
 #pragma unroll
   for (int k = 0; k < NK; ++k) {
