@@ -162,6 +162,10 @@ int stlp_patch_core_pixels(StlpPatchHandle* h, size_t* out);
 int stlp_patch_forward(StlpPatchHandle* h, const double* x, size_t n, uint64_t generation, bool moments, double* out,
                        double* var);
 int stlp_patch_vjp(StlpPatchHandle* h, const double* cot, size_t n, uint64_t generation, double* out);
+/* stlp_patch_forward of patches in memory of their own: parts[i] holds the
+ * sizes[i] values of disc i (no reference counterpart: its caller packs them). */
+int stlp_patch_forward_parts(StlpPatchHandle* h, const double* const* parts, const size_t* sizes, size_t n_parts,
+                             uint64_t generation, bool moments, double* out, double* var);
 int stlp_patch_forward_device(StlpPatchHandle* h, uint64_t x, size_t n, uint64_t generation, bool moments,
                               double* out, double* var);
 int stlp_patch_vjp_device(StlpPatchHandle* h, const double* cot, size_t n, uint64_t generation, uint64_t out);

@@ -21,6 +21,7 @@
 #include "engine.cuh"
 #include "json.hpp"
 #include "lbfgs.hpp"
+#include "hostcopy.hpp"
 #include "scatcov.hpp"
 #include "spin.hpp"
 #include "../../include/stl_b200.h"
@@ -355,8 +356,7 @@ int stlp_forward(StlpHandle* h, const double* x, size_t n, uint64_t generation, 
     require(!moments || var != nullptr, "moments need a variance buffer");
     // small inputs are checked here; larger ones while their copy to the
     // device is staged (load_host), on several host threads
-    if (n < (size_t(1) << 19))
-      for (size_t i = 0; i < n; ++i) require(std::isfinite(x[i]), "input map contains non-finite values");
+    if (n < (size_t(1) << 19)) require(host_nonfinite(x, n) == 0, "input map contains non-finite values");
     h->activate();
     h->has_current = false;
     if (h->spin) h->spin->load_host(*h->engine, x);
@@ -474,7 +474,7 @@ int stlp_forward_levels(StlpHandle* h, const double* x, size_t n, double* out) {
     size_t want = 0;
     for (int d = 0; d < h->engine->levels(); ++d) want += (size_t)h->engine->options().B * h->engine->npix(d);
     require(n == want, "input shape mismatch");
-    for (size_t i = 0; i < n; ++i) require(std::isfinite(x[i]), "input map contains non-finite values");
+    require(host_nonfinite(x, n) == 0, "input map contains non-finite values");
     h->activate();
     h->has_current = false;  // a validation sweep: no vjp or checkpoint follows it
     h->engine->load_levels(x);
@@ -491,7 +491,7 @@ int stlp_spin_fields(StlpHandle* h, const double* x, size_t n, size_t level, dou
     require(n == h->input_len(), "input shape mismatch");
     const int levels = h->spin->config().transported ? h->engine->levels() : 1;
     require(level < (size_t)levels, "level out of range");
-    for (size_t i = 0; i < n; ++i) require(std::isfinite(x[i]), "input map contains non-finite values");
+    require(host_nonfinite(x, n) == 0, "input map contains non-finite values");
     h->activate();
     h->spin->fields(x, (int)level, qu, chi);
     return 0;

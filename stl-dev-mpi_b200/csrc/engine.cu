@@ -106,7 +106,7 @@ void device_bytes_reset_peak() { std::lock_guard<std::mutex> g(g_mem_mu); g_peak
 // (and the reverse for device-to-host), so the transfer runs at the PCIe rate.
 namespace {
 
-// a fixed pool of host threads that split one memcpy between them
+// a fixed pool of host threads that split one copy between them
 class CopyPool {
  public:
   static CopyPool& get() {
@@ -117,19 +117,27 @@ class CopyPool {
   // check (n a multiple of 8): the number of non-finite doubles copied.
   // With widen: src holds n bytes of floats, dst receives them as doubles.
   size_t copy(void* dst, const void* src, size_t n, bool check = false, bool widen = false) {
-    if (n < (size_t(1) << 20) || workers_.empty())
-      return copy_part(static_cast<char*>(dst), static_cast<const char*>(src), n, check, widen);
+    char* d = static_cast<char*>(dst);
+    const char* c = static_cast<const char*>(src);
+    return split(n, [=](size_t lo, size_t hi) -> size_t {
+      if (widen) {  // floats to doubles (exact)
+        host_widen(reinterpret_cast<double*>(d + 2 * lo), reinterpret_cast<const float*>(c + lo), (hi - lo) / 4);
+        return 0;
+      }
+      return host_copy(d + lo, c + lo, hi - lo, check);
+    });
+  }
+  // f(lo, hi) over [0, n) in 64-byte units, by the calling thread and the pool;
+  // the sum of what f returns
+  size_t split(size_t n, const std::function<size_t(size_t, size_t)>& f) {
+    if (n < (size_t(1) << 20) || workers_.empty()) return n ? f(0, n) : 0;
     std::unique_lock<std::mutex> lk(call_mu_);  // one copy at a time
     const size_t parts = workers_.size() + 1;
-    const size_t part = ((n + parts - 1) / parts + 63) & ~(size_t)63;
     {
       std::lock_guard<std::mutex> g(mu_);
-      dst_ = static_cast<char*>(dst);
-      src_ = static_cast<const char*>(src);
+      job_ = &f;
       n_ = n;
-      part_ = part;
-      check_ = check;
-      widen_ = widen;
+      part_ = ((n + parts - 1) / parts + 63) & ~(size_t)63;
       bad_ = 0;
       pending_ = (int)workers_.size();
       ++gen_;
@@ -139,13 +147,6 @@ class CopyPool {
     std::unique_lock<std::mutex> g(mu_);
     done_.wait(g, [&] { return pending_ == 0; });
     return bad_ + b0;
-  }
-  static size_t copy_part(char* dst, const char* src, size_t n, bool check, bool widen = false) {
-    if (widen) {  // floats to doubles (exact)
-      host_widen(reinterpret_cast<double*>(dst), reinterpret_cast<const float*>(src), n / 4);
-      return 0;
-    }
-    return host_copy(dst, src, n, check);
   }
 
  private:
@@ -157,7 +158,7 @@ class CopyPool {
   }
   size_t run(size_t k) {
     const size_t lo = std::min(n_, k * part_), hi = std::min(n_, lo + part_);
-    return hi > lo ? copy_part(dst_ + (widen_ ? 2 * lo : lo), src_ + lo, hi - lo, check_, widen_) : 0;
+    return hi > lo ? (*job_)(lo, hi) : 0;
   }
   void loop(size_t k) {
     uint64_t seen = 0;
@@ -176,10 +177,8 @@ class CopyPool {
   std::vector<std::thread> workers_;
   std::mutex mu_, call_mu_;
   std::condition_variable cv_, done_;
-  char* dst_ = nullptr;
-  const char* src_ = nullptr;
+  const std::function<size_t(size_t, size_t)>* job_ = nullptr;
   size_t n_ = 0, part_ = 0, bad_ = 0;
-  bool check_ = false, widen_ = false;
   int pending_ = 0;
   uint64_t gen_ = 0;
 };
@@ -188,37 +187,43 @@ class CopyPool {
 class HostStage {
  public:
   ~HostStage() {
-    for (cudaEvent_t& e : ev_)
+    for (cudaEvent_t e : {ev_[0], ev_[1], small_ev_})
       if (e) cudaEventDestroy(e);
   }
   // device dst <- host src (n bytes), queued on s; src is read before the
   // return.  With check (src holds doubles): the number of non-finite values.
   size_t to_device(void* dst, const void* src, size_t n, cudaStream_t s, bool check = false) {
-    if (n < kDirect) {
-      size_t bad = 0;
-      if (check) {
-        const double* v = static_cast<const double*>(src);
-        for (size_t i = 0; i < n / 8; ++i) bad += !std::isfinite(v[i]);
-      }
-      STL_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s));
-      return bad;
-    }
-    ensure();
-    size_t bad = 0;
-    for (size_t off = 0, c = 0; off < n; off += kChunk, ++c) {
-      const size_t len = std::min(kChunk, n - off), b = c & 1;
-      STL_CUDA(cudaEventSynchronize(ev_[b]));  // the last DMA out of this buffer has finished
-      bad += CopyPool::get().copy(buf_[b].p, static_cast<const char*>(src) + off, len, check);
-      STL_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + off, buf_[b].p, len, cudaMemcpyHostToDevice, s));
-      STL_CUDA(cudaEventRecord(ev_[b], s));
-    }
-    return bad;
+    return to_device(dst, n, s, [&](char* to, size_t off, size_t len) {
+      return CopyPool::get().copy(to, static_cast<const char*>(src) + off, len, check);
+    });
+  }
+  // the same from parts laid end to end: part i holds doubles at[i] .. at[i + 1]
+  // of the whole, of which [first, first + m) are sent (checked)
+  size_t parts_to_device(void* dst, const double* const* parts, const size_t* at, size_t n_parts, size_t first, size_t m,
+                         cudaStream_t s) {
+    return to_device(dst, m * 8, s, [&](char* to, size_t off, size_t len) {
+      return CopyPool::get().split(len, [&](size_t lo, size_t hi) {
+        size_t p = first + (off + lo) / 8, bad = 0;
+        const size_t end = first + (off + hi) / 8;
+        double* out = reinterpret_cast<double*>(to + lo);
+        size_t i = (size_t)(std::upper_bound(at, at + n_parts + 1, p) - at) - 1;
+        for (; p < end; ++i) {
+          const size_t q = std::min(end, at[i + 1]);
+          if (q > p) bad += host_copy(out, parts[i] + (p - at[i]), (q - p) * 8, true);
+          out += q - p;
+          p = q;
+        }
+        return bad;
+      });
+    });
   }
   // host dst <- device src (n bytes) after the work queued on s; synchronises
   void to_host(void* dst, const void* src, size_t n, cudaStream_t s) {
-    if (n < kDirect) {
-      STL_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, s));
+    if (n < kDirect) {  // through a small pinned buffer
+      void* p = small(n);
+      STL_CUDA(cudaMemcpyAsync(p, src, n, cudaMemcpyDeviceToHost, s));
       STL_CUDA(cudaStreamSynchronize(s));
+      host_copy(dst, p, n, false);
       return;
     }
     ensure();
@@ -241,10 +246,10 @@ class HostStage {
   void to_host_widen(double* dst, const float* src, size_t n, cudaStream_t s) {
     const size_t bytes = n * sizeof(float);
     if (bytes < kDirect) {
-      std::vector<float> tmp(n);
-      STL_CUDA(cudaMemcpyAsync(tmp.data(), src, bytes, cudaMemcpyDeviceToHost, s));
+      float* p = static_cast<float*>(small(bytes));
+      STL_CUDA(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, s));
       STL_CUDA(cudaStreamSynchronize(s));
-      for (size_t i = 0; i < n; ++i) dst[i] = (double)tmp[i];
+      host_widen(dst, p, n);
       return;
     }
     ensure();
@@ -266,6 +271,36 @@ class HostStage {
 
  private:
   static constexpr size_t kChunk = size_t(32) << 20, kDirect = size_t(4) << 20;
+  // n bytes to the device, filled by fill(to, offset, length) in pinned memory:
+  // one small buffer up to kDirect, else the two chunks
+  template <typename F>
+  size_t to_device(void* dst, size_t n, cudaStream_t s, F&& fill) {
+    if (n == 0) return 0;
+    if (n < kDirect) {
+      char* p = static_cast<char*>(small(n));
+      const size_t bad = fill(p, (size_t)0, n);
+      STL_CUDA(cudaMemcpyAsync(dst, p, n, cudaMemcpyHostToDevice, s));
+      STL_CUDA(cudaEventRecord(small_ev_, s));
+      return bad;
+    }
+    ensure();
+    size_t bad = 0;
+    for (size_t off = 0, c = 0; off < n; off += kChunk, ++c) {
+      const size_t len = std::min(kChunk, n - off), b = c & 1;
+      STL_CUDA(cudaEventSynchronize(ev_[b]));  // the last DMA out of this buffer has finished
+      bad += fill(static_cast<char*>(buf_[b].p), off, len);
+      STL_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + off, buf_[b].p, len, cudaMemcpyHostToDevice, s));
+      STL_CUDA(cudaEventRecord(ev_[b], s));
+    }
+    return bad;
+  }
+  // the small pinned buffer, of n bytes at least, once its last copy is done
+  void* small(size_t n) {
+    if (!small_ev_) STL_CUDA(cudaEventCreateWithFlags(&small_ev_, cudaEventDisableTiming));
+    STL_CUDA(cudaEventSynchronize(small_ev_));
+    if (small_.bytes < n) small_.alloc(n);
+    return small_.p;
+  }
   void ensure() {
     if (buf_[0].p) return;
     for (int b = 0; b < 2; ++b) {
@@ -274,8 +309,8 @@ class HostStage {
       STL_CUDA(cudaEventRecord(ev_[b], 0));  // completed: the buffers start free
     }
   }
-  PinnedMem buf_[2];
-  cudaEvent_t ev_[2] = {nullptr, nullptr};
+  PinnedMem buf_[2], small_;
+  cudaEvent_t ev_[2] = {nullptr, nullptr}, small_ev_ = nullptr;
 };
 
 }  // namespace
@@ -786,6 +821,13 @@ class EngineImpl final : public Engine {
     load_maps(in_f64_.as<double>());
   }
 
+  void load_parts(const double* const* parts, const size_t* at, size_t n_parts, size_t first) override {
+    prepare();
+    if (io_.parts_to_device(in_f64_.p, parts, at, n_parts, first, (size_t)opt_.B * npix(0), stream_))
+      throw std::runtime_error("input map contains non-finite values");
+    load_maps(in_f64_.as<double>());
+  }
+
   // level-0 maps (map-major, device) -> constants [B] and pixel-major
   // deviations; the pyramid levels carry the same constants
   template <typename Tin>
@@ -921,15 +963,22 @@ class EngineImpl final : public Engine {
       });
     });
     cudaStream_t s = stream_;
-    STL_CUDA(cudaMemcpyAsync(values, vals_dev_.p, 16 * nv, cudaMemcpyDeviceToHost, s));
-    if (moments && var) STL_CUDA(cudaMemcpyAsync(var, var_dev_.p, 8 * nv, cudaMemcpyDeviceToHost, s));
-    int err = 0;
-    STL_CUDA(cudaMemcpyAsync(&err, err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    // the results through pinned memory with one wait; large ones straight to the
+    // caller's pages (the chunked copy measured no faster for them)
+    const size_t vb = 16 * nv, mb = moments && var ? 8 * nv : 0;
+    const bool pinned = vb + mb <= kPinnedResults;
+    if (pinned && out_pin_.bytes < 8 + vb + mb) out_pin_.alloc(8 + vb + mb);
+    if (!err_pin_.p) err_pin_.alloc(8);
+    char* op = static_cast<char*>(out_pin_.p);
+    STL_CUDA(cudaMemcpyAsync(err_pin_.p, err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    STL_CUDA(cudaMemcpyAsync(pinned ? (void*)op : values, vals_dev_.p, vb, cudaMemcpyDeviceToHost, s));
+    if (mb) STL_CUDA(cudaMemcpyAsync(pinned ? (void*)(op + vb) : var, var_dev_.p, mb, cudaMemcpyDeviceToHost, s));
     STL_CUDA(cudaStreamSynchronize(s));
     prof_.collect();
-    if (err) {
-      STL_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), s));
-      throw std::runtime_error(wait_timeout_message(err, "the forward sweep"));
+    check_error("the forward sweep");
+    if (pinned) {
+      std::memcpy(values, op, vb);
+      if (mb) std::memcpy(var, op + vb, mb);
     }
     forward_done_ = true;
     timers.forward_ms += ms_since(t0);
@@ -1048,7 +1097,10 @@ class EngineImpl final : public Engine {
                    });
   }
 
+  // reverse_impl queues the sweep and the copy of its error flag; the caller
+  // waits for the stream and then checks the flag (finish_reverse)
   void reverse_host(const double* cot, double* out) override {
+    const auto t0 = std::chrono::steady_clock::now();
     reverse_impl(cot);
     i64 n = (i64)opt_.B * npix(0);
     if (!hi(0)) {  // FP32 gradients: moved as floats and widened on the host (exact)
@@ -1056,6 +1108,7 @@ class EngineImpl final : public Engine {
         to_map_major<float, float>(gX_[0].as<float>(), in_f64_.as<float>(), npix(0), opt_.B, stream_);
       });
       io_.to_host_widen(out, in_f64_.as<float>(), (size_t)n, stream_);
+      finish_reverse(t0);
       return;
     }
     prof_.launch(Profiler::ELEM, 1, n * (8.0 + esz(0)), 0.0, stream_, [&] {
@@ -1065,9 +1118,11 @@ class EngineImpl final : public Engine {
       });
     });
     io_.to_host(out, in_f64_.p, n * 8, stream_);
+    finish_reverse(t0);
   }
 
   void reverse_device(const double* cot, void* out, bool f32) override {
+    const auto t0 = std::chrono::steady_clock::now();
     reverse_impl(cot);
     i64 n = (i64)opt_.B * npix(0);
     prof_.launch(Profiler::ELEM, 1, n * ((f32 ? 4.0 : 8.0) + esz(0)), 0.0, stream_, [&] {
@@ -1078,6 +1133,7 @@ class EngineImpl final : public Engine {
       });
     });
     STL_CUDA(cudaStreamSynchronize(stream_));
+    finish_reverse(t0);
   }
 
   size_t host_to_device(void* dst, const void* src, size_t n, bool check) override {
@@ -1087,6 +1143,7 @@ class EngineImpl final : public Engine {
 
   void reverse_levels(const double* cot, double* const* out) override {
     if (!levels_given_) throw std::runtime_error("per-level cotangents need maps given at every level");
+    const auto t0 = std::chrono::steady_clock::now();
     reverse_impl(cot);
     for (int d = 0; d < levels_; ++d)
       prof_.launch(Profiler::ELEM, 1, (double)opt_.B * npix(d) * (8.0 + esz(d)), 0.0, stream_, [&] {
@@ -1096,6 +1153,7 @@ class EngineImpl final : public Engine {
         });
       });
     STL_CUDA(cudaStreamSynchronize(stream_));
+    finish_reverse(t0);
   }
 
   std::vector<KernelStat> kernel_stats() const override {
@@ -1347,22 +1405,28 @@ class EngineImpl final : public Engine {
     reverse_sweep();
   }
 
-  // the reverse sweep from the coefficient cotangents in cot_dev_
+  // queues the reverse sweep from the coefficient cotangents in cot_dev_
   void reverse_sweep() {
-    auto t0 = std::chrono::steady_clock::now();
-    cudaStream_t s = stream_;
     in_graph(grev_, levels_given_ ? 1 : 0, [&] { reverse_launches(); });
-    int err = 0;
-    STL_CUDA(cudaMemcpyAsync(&err, err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    STL_CUDA(cudaStreamSynchronize(s));
+    if (!err_pin_.p) err_pin_.alloc(8);
+    STL_CUDA(cudaMemcpyAsync(err_pin_.p, err_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  }
+  // after the stream was waited for
+  void finish_reverse(std::chrono::steady_clock::time_point t0) {
     prof_.collect();
-    if (err) {
-      STL_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), s));
-      throw std::runtime_error(wait_timeout_message(err, "the reverse sweep"));
-    }
+    check_error("the reverse sweep");
     timers.reverse_ms += ms_since(t0);
     timers.reverses += 1;
   }
+  // the sweep's error flag, copied to err_pin_ on a stream that was waited for
+  void check_error(const char* where) {
+    const int err = *err_pin_.as<int>();
+    if (!err) return;
+    STL_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_));
+    throw std::runtime_error(wait_timeout_message(err, where));
+  }
+  static constexpr size_t kPinnedResults = size_t(4) << 20;
+  PinnedMem out_pin_, err_pin_;
 
   // the reverse launches: cotangent matrices, then the levels descending and
   // the mean / variance terms into gX_[0]

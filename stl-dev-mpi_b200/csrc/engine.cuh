@@ -77,6 +77,7 @@ struct PinnedMem {
   ~PinnedMem() { release(); }
   void alloc(size_t n);
   void release();
+  template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
 // Message of a kernel's timed-out copy wait (the error flag's value: 1 a

@@ -85,6 +85,10 @@ size_t host_copy(void* dst, const void* src, size_t n, bool check) {
   return has_avx() ? copy_avx(d, s, n, check) : copy_scalar(d, s, n, check);
 }
 
+size_t host_nonfinite(const double* x, size_t n) {
+  return count_nonfinite_scalar(reinterpret_cast<const char*>(x), n * 8);
+}
+
 void host_widen(double* dst, const float* src, size_t m) {
   if (has_avx()) {
     widen_avx(dst, src, m);

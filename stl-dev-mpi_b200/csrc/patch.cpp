@@ -457,7 +457,8 @@ int stlp_patch_core_pixels(StlpPatchHandle* h, size_t* out) {
 }
 
 static int patch_forward(StlpPatchHandle* h, const double* x_host, uint64_t x_dev, size_t n, uint64_t generation,
-                         bool moments, double* out, double* var) {
+                         bool moments, double* out, double* var, const double* const* parts = nullptr,
+                         const size_t* at = nullptr) {
   require(h != nullptr && out != nullptr, "null argument");
   require(!moments || var != nullptr, "moments need a variance buffer");
   h->has_current = false;
@@ -466,7 +467,8 @@ static int patch_forward(StlpPatchHandle* h, const double* x_host, uint64_t x_de
   const size_t np = h->plan.size();
   for (auto& g : h->engines()) {  // every group's upload counts non-finite values (load_host)
     Engine& e = *g.engine;
-    if (x_host) e.load_host(x_host + g.offset);
+    if (parts) e.load_parts(parts, at, h->selected.size(), (size_t)g.offset);
+    else if (x_host) e.load_host(x_host + g.offset);
     else e.load_device(reinterpret_cast<const double*>(x_dev) + g.offset, false);
     e.forward(moments, out + 2 * g.first * np, moments ? var + g.first * np : nullptr);
   }
@@ -480,6 +482,22 @@ int stlp_patch_forward(StlpPatchHandle* h, const double* x, size_t n, uint64_t g
   return guard<int>(-1, [&] {
     require(x != nullptr, "null argument");
     return patch_forward(h, x, 0, n, generation, moments, out, var);
+  });
+}
+
+int stlp_patch_forward_parts(StlpPatchHandle* h, const double* const* parts, const size_t* sizes, size_t n_parts,
+                             uint64_t generation, bool moments, double* out, double* var) {
+  return guard<int>(-1, [&] {
+    require(h != nullptr && parts != nullptr && sizes != nullptr, "null argument");
+    require(!h->selected.empty(), "no disc selected");
+    require(n_parts == h->selected.size(), "one part per selected disc expected");
+    std::vector<size_t> at(n_parts + 1, 0);
+    for (size_t i = 0; i < n_parts; ++i) {
+      require(sizes[i] == h->size(i), "input shape mismatch");
+      require(parts[i] != nullptr, "null argument");
+      at[i + 1] = at[i] + sizes[i];
+    }
+    return patch_forward(h, nullptr, 0, at[n_parts], generation, moments, out, var, parts, at.data());
   });
 }
 

@@ -126,6 +126,9 @@ class Engine {
   virtual void prepare() = 0;
   // Loads maps [B][N_0] from host (f64) or device memory (f64 or f32).
   virtual void load_host(const double* x) = 0;
+  // load_host of host parts laid end to end (part i: doubles at[i] .. at[i + 1] of
+  // the whole, n_parts + 1 offsets), from double `first` of the whole on
+  virtual void load_parts(const double* const* parts, const size_t* at, size_t n_parts, size_t first) = 0;
   virtual void load_device(const void* x, bool f32) = 0;
   // Maps given at every level (host f64, the concatenation over d of
   // [B][npix(d)]): the next forward uses them instead of the decimation

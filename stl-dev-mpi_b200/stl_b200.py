@@ -84,6 +84,7 @@ def lib():
             "stlp_patch_ids": ([_VOID, sz, C.POINTER(C.c_int64)], C.c_int),
             "stlp_patch_core_pixels": ([_VOID, _SIZE], C.c_int),
             "stlp_patch_forward": ([_VOID, _D, sz, u64, b, _D, _D], C.c_int),
+            "stlp_patch_forward_parts": ([_VOID, C.POINTER(_VOID), _SIZE, sz, u64, b, _D, _D], C.c_int),
             "stlp_patch_vjp": ([_VOID, _D, sz, u64, _D], C.c_int),
             "stlp_patch_forward_device": ([_VOID, u64, sz, u64, b, _D, _D], C.c_int),
             "stlp_patch_vjp_device": ([_VOID, _D, sz, u64, u64], C.c_int),
@@ -867,7 +868,7 @@ class PatchEngine:
         self.levels = info["levels"]
         self._native = np.array([c["native_dg"] for c in self.plan], dtype=np.int64)
         self.ids, self._selection, self._generation, self._dense = [], None, None, False
-        self._xbuf = None  # the packed patches of the current selection
+        self._sizes, self._cuts = np.zeros(0, np.uintp), np.zeros(0, np.int64)  # of the current selection
 
     def _open(self):
         if not self._handle:
@@ -930,6 +931,7 @@ class PatchEngine:
             if self._lib.stlp_patch_core_pixels(self._handle, per_level.ctypes.data_as(_SIZE)):
                 raise _error()
             self.native_pixels = per_level.astype(np.float64)[:, self._native]
+            self._sizes, self._cuts = counts, np.cumsum(counts.astype(np.int64))
             self._selection = ident
             return self.ids
 
@@ -947,24 +949,17 @@ class PatchEngine:
             return [m[i] for i in self.ids]
         return [m[k][..., i] for k, i in enumerate(self.ids)]
 
-    def _pack(self, maps):
-        """One float64 vector of the patches in disc order, checked against the
-        selection's pixel counts."""
+    def _parts(self, maps):
+        """The patches as float64 vectors in disc order, checked against the
+        selection's pixel counts, with their addresses and sizes for the library
+        (which gathers them while it copies them)."""
         if len(maps) != len(self.ids):
             raise ValueError(f"{len(maps)} patches given for {len(self.ids)} selected discs")
-        sizes = [i.size for i in self.ids]
-        flat = [np.asarray(m, dtype=np.float64) for m in maps]
-        for i, (m, size) in enumerate(zip(flat, sizes)):
+        flat = [np.ascontiguousarray(m, dtype=np.float64) for m in maps]
+        for i, (m, size) in enumerate(zip(flat, self._sizes)):
             if m.shape != (size,):
                 raise ValueError(f"patch {i} has shape {m.shape}; its disc holds {size} pixels")
-        if not flat:
-            return np.zeros(0)
-        # one buffer per selection, reused: the library has read it when the
-        # call returns, and fresh memory would cost its page faults every call
-        total = sum(sizes)
-        if self._xbuf is None or self._xbuf.size != total:
-            self._xbuf = np.empty(total, dtype=np.float64)
-        return np.concatenate(flat, out=self._xbuf)
+        return flat, (_VOID * len(flat))(*[m.ctypes.data for m in flat])
 
     def forward(self, maps, centres=None, radius=None, core=None, moments=True, generation=0, out=None):
         """Statistics [B, ncoeff] (and variances, or [B, 0]) of the patches of
@@ -979,7 +974,7 @@ class PatchEngine:
                 self.select(centres, radius, core)
             if not self.ids:
                 raise RuntimeError("forward before any disc was selected")
-            x = self._pack(maps)  # non-finite values are counted by the library's copy (ValueError)
+            flat, parts = self._parts(maps)  # non-finite values are counted by the library's copy (ValueError)
             b = len(self.ids)
             if out is None:
                 values = np.empty((b, self.ncoeff), dtype=np.complex128)
@@ -991,8 +986,9 @@ class PatchEngine:
             variance = np.empty((b, self.ncoeff if moments else 0), dtype=np.float64)
             self._generation = None
             self._dense = isinstance(maps, np.ndarray)
-            status = self._lib.stlp_patch_forward(self._handle, _ptr(x), x.size, int(generation), bool(moments),
-                                                  _ptr(values.view(np.float64)), _ptr(variance) if moments else None)
+            status = self._lib.stlp_patch_forward_parts(self._handle, parts, self._sizes.ctypes.data_as(_SIZE), b,
+                                                        int(generation), bool(moments), _ptr(values.view(np.float64)),
+                                                        _ptr(variance) if moments else None)
             if status:
                 raise _error()
             self._generation = int(generation)
@@ -1014,8 +1010,7 @@ class PatchEngine:
                 raise ValueError(f"cotangents have shape {c.shape}, the statistics {(b, self.ncoeff)}")
             if not _all_finite(c):
                 raise ValueError("non-finite coefficient cotangent")
-            sizes = np.array([i.size for i in self.ids], dtype=np.int64)
-            total = int(sizes.sum())
+            total = int(self._cuts[-1])
             if out is None:
                 grad = np.empty(total, dtype=np.float64)
             else:
@@ -1026,7 +1021,8 @@ class PatchEngine:
             if self._lib.stlp_patch_vjp(self._handle, _ptr(c.view(np.float64)), c.size, int(generation),
                                         _ptr(grad)):
                 raise _error()
-            parts = np.split(grad, np.cumsum(sizes)[:-1])
+            ends = self._cuts.tolist()
+            parts = [grad[i:j] for i, j in zip([0] + ends[:-1], ends)]
             return np.stack(parts) if self._dense else parts
 
     def close(self):
