@@ -287,6 +287,30 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const int32_t* __restrict__ ce
     for (int rb = 0; rb < RB; ++rb)
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[k][rb][j] = (T)0;
+  if constexpr (NK == 1) {
+    // Grid operators: SB slots at a time.  The cells of the next batch are loaded
+    // with this batch's coefficients and values, so SB gathers and coefficient
+    // rows are in flight a thread (one slot ahead: 7.74 ms a forward of 512 discs of
+    // nside 512, J 5, FP32, now 6.36; 13 FP64 discs of nside 128, J 4 0.28 -> 0.22).  Past the last slot its loads are repeated and not used.
+    constexpr int SB = sizeof(T) == 4 ? 4 : 2;
+    i64 c[SB];
+#pragma unroll
+    for (int j = 0; j < SB; ++j) c[j] = __ldg(cell + (i64)min(j, S - 1) * n_rep + u);
+    for (int s = 0; s < S; s += SB) {
+      T xv[SB][RB], w[SB][8];
+#pragma unroll
+      for (int j = 0; j < SB; ++j) {
+        loadR<RB>(x + c[j] * R + r0, xv[j]);
+        load8(coef + ((i64)min(s + j, S - 1) * n_rep + u) * 8, w[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < SB; ++j) c[j] = __ldg(cell + (i64)min(s + SB + j, S - 1) * n_rep + u);
+#pragma unroll
+      for (int j = 0; j < SB; ++j) {
+        if (s + j < S) fma_rows<RB>(acc[0], w[j], xv[j]);
+      }
+    }
+  } else {
   // Two-stage software pipeline: the gathers of slot s + 1 and the cell of
   // slot s + 2 are in flight while slot s is accumulated.
   T xv[NK][RB], xn[NK][RB], w[8], wn[8];
@@ -315,6 +339,7 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const int32_t* __restrict__ ce
       for (int rb = 0; rb < RB; ++rb) xv[k][rb] = xn[k][rb];
 #pragma unroll
     for (int j = 0; j < 8; ++j) w[j] = wn[j];
+  }
   }
   if (rc) {  // the rows' constants times the row sums of the coefficients
     T rs[8];
@@ -560,7 +585,7 @@ __global__ void __launch_bounds__(128) k_conv_adj(const uint32_t* __restrict__ t
 #pragma unroll
     for (int rb = 0; rb < RB; ++rb) acc[k][rb] = (T)0;
   if (NK == 1) {
-    // Grid operators: a two-stage software pipeline, as in k_conv_fwd: the
+    // Grid operators: a two-stage software pipeline: the
     // coefficients and cotangent rows of entry q + 1 and the entry index of
     // q + 2 are in flight while entry q is added (entries in order).
     T w[8], g[RB][8], wn[8], gn[RB][8];
