@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const int32_t* __restrict__ ce
     // Grid operators: SB slots at a time.  The cells of the next batch are loaded
     // with this batch's coefficients and values, so SB gathers and coefficient
     // rows are in flight a thread (one slot ahead: 7.74 ms a forward of 512 discs of
-    // nside 512, J 5, FP32, now 6.36; 13 FP64 discs of nside 128, J 4 0.28 -> 0.22).  Past the last slot its loads are repeated and not used.
+    // nside 512, J 5, FP32, now 6.36; 13 FP64 discs of nside 128, J 4 0.28 -> 0.22).  Past
+    // the last slot its loads are repeated and not used.
     constexpr int SB = sizeof(T) == 4 ? 4 : 2;
     i64 c[SB];
 #pragma unroll
