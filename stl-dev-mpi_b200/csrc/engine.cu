@@ -716,8 +716,6 @@ class EngineImpl final : public Engine {
     shapes_.resize(levels_);
     size_t max_part = 0, max_gz = 0, max_gbr = 0, coarse_gz = 0, coarse_gbr = 0;
     part_off_.clear();
-    gz_off_.clear();
-    gbr_off_.clear();
     // field store: z and the branches of every level kept, or one buffer each
     // (the largest level's) recomputed per level in the reverse sweep
     {
@@ -759,11 +757,9 @@ class EngineImpl final : public Engine {
       const size_t gz = e * 2 * B * L * N, gbr = e * 2 * B * (n + 1) * L * L * N;
       max_gz = std::max(max_gz, gz);
       max_gbr = std::max(max_gbr, gbr);
-      gz_off_.push_back(coarse_gz);  // levels above 0: buffers of their own
-      gbr_off_.push_back(coarse_gbr);
       if (n > 0) {
-        coarse_gz += (gz + 255) & ~(size_t)255;
-        coarse_gbr += (gbr + 255) & ~(size_t)255;
+        coarse_gz = std::max(coarse_gz, gz);
+        coarse_gbr = std::max(coarse_gbr, gbr);
       }
       field_bytes_ += X_[n].bytes + Z_[n].bytes + Mod_[n].bytes + Br_[n].bytes + gMod_[n].bytes + gX_[n].bytes;
     }
@@ -794,22 +790,16 @@ class EngineImpl final : public Engine {
     size_mask_buffers();
     gZ_.alloc(max_gz);
     gBr_.alloc(max_gbr);
-    // cotangents of every level of their own and partial sums for the adjoints of
-    // z, so that the products VJPs and the map cotangents run beside the chain of
-    // the moduli (0.8 of the level-0 buffers; left out when they would take a
-    // quarter of the free memory)
+    // cotangents of the coarser levels of their own, so that the products VJP of
+    // level 0 runs beside those levels (half the level-0 buffers; left out when
+    // they would take a quarter of the free memory)
     if (forks() && levels_ > 1) {
-      size_t cap = 0;
-      for (int n = 0; n < levels_; ++n) cap = std::max(cap, adjoint_part_bytes(conv_[n], esz(n), B));
       size_t free_b = 0, total_b = 0;
       STL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      if (coarse_gz + coarse_gbr + cap < free_b / 4) {
+      if (coarse_gz + coarse_gbr < free_b / 4) {
         gZc_.alloc(coarse_gz);
         gBrc_.alloc(coarse_gbr);
-        if (cap) adjz_part_.alloc(cap);
-        adjz_.part = adjz_part_.p;
-        adjz_.capacity = cap;
-        field_bytes_ += gZc_.bytes + gBrc_.bytes + adjz_part_.bytes;
+        field_bytes_ += gZc_.bytes + gBrc_.bytes;
       }
     }
     err_.alloc(sizeof(int));
@@ -819,7 +809,7 @@ class EngineImpl final : public Engine {
     xc_.alloc(sizeof(double) * levels_ * B);
     zc_.alloc(sizeof(double) * levels_ * B * L);
     rc_.alloc(sizeof(double) * B * levels_ * L * levels_);  // a set per level
-    mpart_.alloc(sizeof(double) * kMeansBlocks * B * L * levels_);  // a set per level
+    mpart_.alloc(sizeof(double) * kMeansBlocks * B * L);
     in_f64_.alloc(sizeof(double) * B * npix(0));
     field_bytes_ += partials_.bytes + sums_.bytes + gZ_.bytes + gBr_.bytes + in_f64_.bytes;
     if (!hi(0)) {  // FP32 level 0: the rounding residuals of its deviations
@@ -1017,14 +1007,10 @@ class EngineImpl final : public Engine {
   }
 
   // the forward launches: pyramid, then every level's fields and sums
-  // Three chains: the map pyramid with every level's z, its moduli and their
-  // means (fork z_side(n)); the stored moduli pushed down level by level; the
-  // branches and products (fork n).  On one stream level by level, so that
-  // levels may share the buffers of z and the branches (recomputed fields).
   void forward_sweep(bool moments) {
     const int B = opt_.B;
-    auto pyramid = [&](int d) {
-      cudaStream_t s = stream_;
+    cudaStream_t s = stream_;
+    for (int d = 0; d + 1 < levels_ && !levels_given_; ++d)
       prof_.launch(Profiler::DEC, 1, dec_bytes(dec_[d], B, false), dec_flops(dec_[d], B, false), s, [&] {
         typed(d, [&](auto ti) {
           typed(d + 1, [&](auto to) {
@@ -1035,19 +1021,8 @@ class EngineImpl final : public Engine {
           });
         });
       });
-    };
-    auto z = [&](int n) { typed(n, [&](auto t) { forward_z<typename decltype(t)::type>(n); }); };
-    const bool apart = forks() && !prof_.on;
-    for (int d = 0; d < levels_; ++d) {
-      if (apart) fork(z_side(d), [&] { z(d); });
-      if (d + 1 < levels_ && !levels_given_) pyramid(d);
-    }
-    for (int n = 0; n < levels_; ++n) {
-      if (apart) join(z_side(n));
-      else z(n);
-      typed(n, [&](auto t) { forward_moduli<typename decltype(t)::type>(n); });
-      fork(n, [&] { typed(n, [&](auto t) { forward_branches<typename decltype(t)::type>(n, moments); }); });
-    }
+    for (int n = 0; n < levels_; ++n)
+      typed(n, [&](auto t) { forward_level<typename decltype(t)::type>(n, moments); });
     join();
   }
 
@@ -1089,9 +1064,8 @@ class EngineImpl final : public Engine {
 
   int* error_flag() override { return err_.as<int>(); }
 
-  // z of level n, and |z| into slot n of the level's stored moduli
   template <typename U>
-  void forward_z(int n) {
+  void forward_level(int n, bool moments) {
     const int L = opt_.L, B = opt_.B;
     cudaStream_t s = stream_;
     const i64 N = npix(n);
@@ -1104,17 +1078,9 @@ class EngineImpl final : public Engine {
     // |z| as deviations from their means per (map, orientation)
     double* zc = zc_.as<double>() + (size_t)n * B * L;
     prof_.launch(Profiler::ELEM, 3, (double)N * B * L * (2 * 2 * sizeof(U) + sizeof(U)), 0.0, s, [&] {
-      row_means<U>(zf<U>(n), true, true, N, B * L, mpart_.as<double>() + (size_t)n * kMeansBlocks * B * L, zc, s);
+      row_means<U>(zf<U>(n), true, true, N, B * L, mpart_.as<double>(), zc, s);
       moduli_deviations<U>(zf<U>(n), N, B, L, zc, mod, B * (n + 1) * L, (n + 1) * L, n * L, s);
     });
-  }
-
-  // the finer levels' stored moduli pushed down into level n
-  template <typename U>
-  void forward_moduli(int n) {
-    const int L = opt_.L, B = opt_.B;
-    cudaStream_t s = stream_;
-    U* mod = Mod_[n].as<U>();
     if (n > 0)
       prof_.launch(Profiler::DEC, 1, dec_bytes(dec_[n - 1], B * n * L, false), dec_flops(dec_[n - 1], B * n * L, false),
                    s, [&] {
@@ -1124,6 +1090,8 @@ class EngineImpl final : public Engine {
                                         B * (n + 1) * L, (n + 1) * L, B, n * L, false, s, tile(n, T_DEC_MOD));
                      });
                    });
+    // the next level needs this level's moduli only: its branches and products run beside it
+    fork(n, [&] { forward_branches<U>(n, moments); });
   }
 
   // the second wavelets of level n and its coefficient sums
@@ -1503,8 +1471,7 @@ class EngineImpl final : public Engine {
     cudaStream_t s = stream_;
     // per level and mask: cotangent matrices and S1 scales in the level's
     // field type; the mean and variance scales
-    auto matrices = [&](int n) {
-      cudaStream_t s = stream_;
+    for (int n = 0; n < levels_; ++n)
       prof_.launch(Profiler::ELEM, 1, (double)K_ * B * (L * shapes_[n].K * shapes_[n].K + L) * 16.0, 0.0, s, [&] {
         typed(n, [&](auto t) {
           using U = typename decltype(t)::type;
@@ -1516,25 +1483,15 @@ class EngineImpl final : public Engine {
                               reinterpret_cast<U*>(base + stage_s_[(size_t)n * K_]), s, opt_.cross);
         });
       });
-    };
-    const bool apart = gBrc_.p && !prof_.on;
-    if (apart) {  // every level's products VJP, the coarsest first, beside the chain of the moduli
-      for (int n = levels_ - 1; n >= 0; --n)
-        fork(n, [&] {
-          matrices(n);
-          typed(n, [&](auto t) { reverse_products<typename decltype(t)::type>(n); });
-        });
-    } else {
-      for (int n = 0; n < levels_; ++n) matrices(n);
-    }
     if (!opt_.cross)
       prof_.launch(Profiler::ELEM, 1, 16.0 * B * K_ * 2, 0.0, s, [&] {
         build_mean_var(cot_dev_.as<double>(), np, B, K_, counts_dev_.as<double>(), levels_, i_mean_, i_var_,
                        mv_.as<double>(), s);
       });
+    if (gBrc_.p)  // level 0's products VJP beside the coarser levels
+      fork(0, [&] { typed(0, [&](auto t) { reverse_products<typename decltype(t)::type>(0); }); });
     for (int n = levels_ - 1; n >= 0; --n)
-      typed(n, [&](auto t) { reverse_level<typename decltype(t)::type>(n, apart); });
-    join();
+      typed(n, [&](auto t) { reverse_level<typename decltype(t)::type>(n); });
     for (int k = 0; k < launch_sets() && !opt_.cross; ++k)  // the cross plan has no mean or variance
       prof_.launch(Profiler::ELEM, 1, (double)B * npix(0) * 3 * esz(0), (double)B * npix(0) * 2.0, s, [&] {
         typed(0, [&](auto t) {
@@ -1574,7 +1531,7 @@ class EngineImpl final : public Engine {
   // one level of the reverse sweep (field type U); M: the level's cotangent
   // matrices [B][L][K][K], s1: the auto-S1 scales [B][L]
   template <typename U>
-  void reverse_level(int n, bool apart) {
+  void reverse_level(int n) {
     const int L = opt_.L, B = opt_.B;
     cudaStream_t s = stream_;
     const i64 N = npix(n);
@@ -1608,7 +1565,7 @@ class EngineImpl final : public Engine {
       });
     }
     const double sz = sizeof(U);
-    if (apart) join((size_t)n);
+    if (n == 0 && gBrc_.p) join();
     else reverse_products<U>(n);
     const int R = B * (n + 1) * L;
     prof_.launch(Profiler::CONV_ADJ, adjoint_tiles_usable(op, sizeof(U), R, adj_ptr()) ? 2 : 1,
@@ -1617,20 +1574,6 @@ class EngineImpl final : public Engine {
                    conv_adjoint<U>(op, gbrf<U>(n), R, gmod, true, s, adj_ptr(), err_.as<int>(), nullptr,
                                    tile(n, T_ADJ_BR));
                  });
-    // the next level needs this level's moduli only: the map cotangents run beside it
-    if (apart) fork(x_side(), [&] { reverse_maps<U>(n, adjz_ptr()); });
-    else reverse_maps<U>(n, adj_ptr());
-  }
-
-  // the adjoint of z of level n into its map cotangent, plus the next level's
-  template <typename U>
-  void reverse_maps(int n, const AdjScratch* scratch) {
-    const int L = opt_.L, B = opt_.B;
-    cudaStream_t s = stream_;
-    const i64 N = npix(n);
-    const ConvOp& op = conv_[n];
-    U* gmod = gMod_[n].as<U>();
-    const double sz = sizeof(U);
     // the modulus VJP of z (gZ += gmod z / |z|): inside the coloured adjoint
     // of z when the operator has it, else its own pass
     ModulusAdd<U> madd;
@@ -1638,14 +1581,14 @@ class EngineImpl final : public Engine {
     madd.g = gmod + n * L;
     madd.g_pix = B * (n + 1) * L;
     madd.g_row = (n + 1) * L;
-    const bool fuse = conv_adjoint_fuses_modulus(op, sizeof(U), B, scratch, err_.as<int>());
+    const bool fuse = conv_adjoint_fuses_modulus(op, sizeof(U), B, adj_ptr(), err_.as<int>());
     if (!fuse)
       prof_.launch(Profiler::ELEM, 1, (double)B * L * N * 5 * sz, (double)B * L * N * 6.0, s, [&] {
         modulus_vjp_add<U>(zf<U>(n), gmod + n * L, B * (n + 1) * L, (n + 1) * L, gzf<U>(n), N, B, L, s);
       });
-    prof_.launch(Profiler::CONV_ADJ, adjoint_tiles_usable(op, sizeof(U), B, scratch) ? 2 : 1,
+    prof_.launch(Profiler::CONV_ADJ, adjoint_tiles_usable(op, sizeof(U), B, adj_ptr()) ? 2 : 1,
                  conv_bytes(op, B, false, false), conv_flops(op, B), s, [&] {
-                   conv_adjoint<U>(op, gzf<U>(n), B, gX_[n].as<U>(), false, s, scratch, err_.as<int>(),
+                   conv_adjoint<U>(op, gzf<U>(n), B, gX_[n].as<U>(), false, s, adj_ptr(), err_.as<int>(),
                                    fuse ? &madd : nullptr, tile(n, T_ADJ_Z));
                  });
     if (n + 1 < levels_ && !levels_given_)  // maps given per level: no chain through the decimation
@@ -1849,7 +1792,7 @@ class EngineImpl final : public Engine {
   // to streams of their own (captured as parallel branches of the sweep's
   // graph), so that the short kernels of the coarse levels run beside the long
   // ones of the fine: fork(i, f) runs f after the work queued so far, on side
-  // stream i; join makes the sweep's stream wait for side stream i, or for all.
+  // stream i; join() makes the sweep's stream wait for every side stream used.
   // One stream where the sweeps run kernel by kernel ("graphs": false,
   // profiling) and where levels share buffers (recomputed fields).
   std::vector<cudaStream_t> side_;
@@ -1857,27 +1800,26 @@ class EngineImpl final : public Engine {
   std::vector<char> side_used_;
   bool forks() const { return opt_.graphs && !recompute_; }
   template <typename F>
-  void fork(size_t i, F&& f) {
+  void fork(int i, F&& f) {
     if (!forks() || prof_.on) {
       f();
       return;
     }
     if (side_.empty()) {
-      const int sides = 2 * levels_ + 1;
-      for (int k = 0; k <= sides; ++k) {
+      for (int k = 0; k <= levels_; ++k) {
         cudaEvent_t e;
         STL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         side_ev_.push_back(e);
-        if (k == sides) break;
+        if (k == levels_) break;
         cudaStream_t st;
         STL_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         side_.push_back(st);
       }
-      side_used_.assign(sides, 0);
+      side_used_.assign(levels_, 0);
     }
     cudaStream_t main = stream_;
-    STL_CUDA(cudaEventRecord(side_ev_.back(), main));
-    STL_CUDA(cudaStreamWaitEvent(side_[i], side_ev_.back(), 0));
+    STL_CUDA(cudaEventRecord(side_ev_[levels_], main));
+    STL_CUDA(cudaStreamWaitEvent(side_[i], side_ev_[levels_], 0));
     side_used_[i] = 1;
     stream_ = side_[i];
     try {
@@ -1888,31 +1830,18 @@ class EngineImpl final : public Engine {
     }
     stream_ = main;
   }
-  void join(size_t i) {
-    if (i >= side_used_.size() || !side_used_[i]) return;
-    STL_CUDA(cudaEventRecord(side_ev_[i], side_[i]));
-    STL_CUDA(cudaStreamWaitEvent(stream_, side_ev_[i], 0));
-    side_used_[i] = 0;
-  }
   void join() {
-    for (size_t i = 0; i < side_used_.size(); ++i) join(i);
+    for (size_t i = 0; i < side_used_.size(); ++i)
+      if (side_used_[i]) {
+        STL_CUDA(cudaEventRecord(side_ev_[i], side_[i]));
+        STL_CUDA(cudaStreamWaitEvent(stream_, side_ev_[i], 0));
+        side_used_[i] = 0;
+      }
   }
-  // side streams: n the branches or the products VJP of level n, then the z of
-  // level n, then the map cotangents
-  size_t z_side(int n) const { return (size_t)(levels_ + n); }
-  size_t x_side() const { return (size_t)(2 * levels_); }
   std::vector<size_t> part_off_;  // partial sums of every level (doubles)
   DevMem gZc_, gBrc_;             // cotangents of the levels above 0, or none
-  std::vector<size_t> gz_off_, gbr_off_;
-  template <typename U> U* gzf(int n) {
-    return n > 0 && gZc_.p ? reinterpret_cast<U*>(gZc_.as<char>() + gz_off_[n]) : gZ_.as<U>();
-  }
-  template <typename U> U* gbrf(int n) {
-    return n > 0 && gBrc_.p ? reinterpret_cast<U*>(gBrc_.as<char>() + gbr_off_[n]) : gBr_.as<U>();
-  }
-  DevMem adjz_part_;  // partial sums of the adjoints of z beside those of the branches
-  AdjScratch adjz_;
-  const AdjScratch* adjz_ptr() const { return adjz_.part ? &adjz_ : adj_ptr(); }
+  template <typename U> U* gzf(int n) { return n > 0 && gZc_.p ? gZc_.as<U>() : gZ_.as<U>(); }
+  template <typename U> U* gbrf(int n) { return n > 0 && gBrc_.p ? gBrc_.as<U>() : gBr_.as<U>(); }
   double* rc(int n) { return rc_.as<double>() + (size_t)n * opt_.B * levels_ * opt_.L; }
 
   // recompute field store: the one z and branch buffer of every level
