@@ -548,8 +548,6 @@ class EngineImpl final : public Engine {
     gfwd_.reset();
     grev_.reset();
     if (capture_stream_) cudaStreamDestroy(capture_stream_);
-    for (cudaStream_t st : side_) cudaStreamDestroy(st);
-    for (cudaEvent_t e : side_ev_) cudaEventDestroy(e);
   }
   explicit EngineImpl(const Options& o, const Support* sup = nullptr) : Engine(o, sup) {
     int K0 = 0;
@@ -714,8 +712,7 @@ class EngineImpl final : public Engine {
     X_.resize(levels_); Z_.resize(levels_); Mod_.resize(levels_); Br_.resize(levels_);
     gMod_.resize(levels_); gX_.resize(levels_);
     shapes_.resize(levels_);
-    size_t max_part = 0, max_gz = 0, max_gbr = 0, coarse_gz = 0, coarse_gbr = 0;
-    part_off_.clear();
+    size_t max_part = 0, max_gz = 0, max_gbr = 0;
     // field store: z and the branches of every level kept, or one buffer each
     // (the largest level's) recomputed per level in the reverse sweep
     {
@@ -750,17 +747,11 @@ class EngineImpl final : public Engine {
       gX_[n].alloc(e * B * N);
       shapes_[n] = product_shape(n, L, B, N, e);
       if (segmented()) segment_ranges(shapes_[n], support_.seg[n]);
-      // partial sums per level: the products of several levels may run at once
-      part_off_.push_back(max_part);
-      max_part += std::max((size_t)B * L * shapes_[n].blocks * shapes_[n].slots,
-                           opt_.cross ? (size_t)cross_blocks(N) * vb_ * L * cross_slots(shapes_[n].K) : 0);
-      const size_t gz = e * 2 * B * L * N, gbr = e * 2 * B * (n + 1) * L * L * N;
-      max_gz = std::max(max_gz, gz);
-      max_gbr = std::max(max_gbr, gbr);
-      if (n > 0) {
-        coarse_gz = std::max(coarse_gz, gz);
-        coarse_gbr = std::max(coarse_gbr, gbr);
-      }
+      max_part = std::max(max_part, (size_t)B * L * shapes_[n].blocks * shapes_[n].slots);
+      if (opt_.cross)
+        max_part = std::max(max_part, (size_t)cross_blocks(N) * vb_ * L * cross_slots(shapes_[n].K));
+      max_gz = std::max(max_gz, e * 2 * B * L * N);
+      max_gbr = std::max(max_gbr, e * 2 * B * (n + 1) * L * L * N);
       field_bytes_ += X_[n].bytes + Z_[n].bytes + Mod_[n].bytes + Br_[n].bytes + gMod_[n].bytes + gX_[n].bytes;
     }
     partials_.alloc(sizeof(double) * max_part);
@@ -790,25 +781,13 @@ class EngineImpl final : public Engine {
     size_mask_buffers();
     gZ_.alloc(max_gz);
     gBr_.alloc(max_gbr);
-    // cotangents of the coarser levels of their own, so that the products VJP of
-    // level 0 runs beside those levels (half the level-0 buffers; left out when
-    // they would take a quarter of the free memory)
-    if (forks() && levels_ > 1) {
-      size_t free_b = 0, total_b = 0;
-      STL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      if (coarse_gz + coarse_gbr < free_b / 4) {
-        gZc_.alloc(coarse_gz);
-        gBrc_.alloc(coarse_gbr);
-        field_bytes_ += gZc_.bytes + gBrc_.bytes;
-      }
-    }
     err_.alloc(sizeof(int));
     STL_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_));
     // per-row constants of the fields: maps [level][B], moduli [level][B][L],
     // branch rows of one level, and the partial sums of their means
     xc_.alloc(sizeof(double) * levels_ * B);
     zc_.alloc(sizeof(double) * levels_ * B * L);
-    rc_.alloc(sizeof(double) * B * levels_ * L * levels_);  // a set per level
+    rc_.alloc(sizeof(double) * B * levels_ * L);
     mpart_.alloc(sizeof(double) * kMeansBlocks * B * L);
     in_f64_.alloc(sizeof(double) * B * npix(0));
     field_bytes_ += partials_.bytes + sums_.bytes + gZ_.bytes + gBr_.bytes + in_f64_.bytes;
@@ -1023,7 +1002,6 @@ class EngineImpl final : public Engine {
       });
     for (int n = 0; n < levels_; ++n)
       typed(n, [&](auto t) { forward_level<typename decltype(t)::type>(n, moments); });
-    join();
   }
 
   void set_objective(const double* target, const double* weights) override {
@@ -1090,23 +1068,11 @@ class EngineImpl final : public Engine {
                                         B * (n + 1) * L, (n + 1) * L, B, n * L, false, s, tile(n, T_DEC_MOD));
                      });
                    });
-    // the next level needs this level's moduli only: its branches and products run beside it
-    fork(n, [&] { forward_branches<U>(n, moments); });
-  }
-
-  // the second wavelets of level n and its coefficient sums
-  template <typename U>
-  void forward_branches(int n, bool moments) {
-    const int L = opt_.L, B = opt_.B;
-    cudaStream_t s = stream_;
-    const i64 N = npix(n);
-    U* mod = Mod_[n].as<U>();
-    const ConvOp& op = conv_[n];
     const int R = B * (n + 1) * L;
     prof_.launch(Profiler::ELEM, 1, 16.0 * B * L, 0.0, s,
-                 [&] { branch_constants(zc_.as<double>(), n, B, L, rc(n), s); });
+                 [&] { branch_constants(zc_.as<double>(), n, B, L, rc_.as<double>(), s); });
     prof_.launch(Profiler::CONV_FWD, 1, conv_bytes(op, R, true, false), conv_flops(op, R), s, [&] {
-      conv_forward<U>(op, mod, R, brf<U>(n), nullptr, 0, 0, 0, s, err_.as<int>(), rc(n),
+      conv_forward<U>(op, mod, R, brf<U>(n), nullptr, 0, 0, 0, s, err_.as<int>(), rc_.as<double>(),
                       tile(n, T_FWD_BR));
     });
     const ProductShape& sh = shapes_[n];
@@ -1116,7 +1082,7 @@ class EngineImpl final : public Engine {
         prof_.launch(Profiler::PROD_FWD, 2, (double)B * L * N * sh.K * 2 * sizeof(U),
                      (double)vb_ * L * N * sh.K * sh.K * 8.0, s, [&] {
                        cross_forward<U>(sh.K, N, B, zf<U>(n), brf<U>(n), mask(k, n), moments,
-                                        partials_.as<double>() + part_off_[n], cross_blocks(N),
+                                        partials_.as<double>(), cross_blocks(N),
                                         sums_.as<double>() + k * total_sums_ + sum_off_[n], s);
                      });
       return;
@@ -1125,8 +1091,7 @@ class EngineImpl final : public Engine {
       prof_.launch(Profiler::PROD_FWD, 2, (double)B * L * N * sh.K * 2 * sizeof(U), (double)B * L * N * E * 10.0, s,
                    [&] {
                      products_forward<U>(sh, zf<U>(n), brf<U>(n), n == 0 ? X_[0].as<U>() : nullptr,
-                                         n == 0 ? xr_.as<U>() : nullptr, xc_.as<double>(), mask(k, n),
-                                         partials_.as<double>() + part_off_[n],
+                                         n == 0 ? xr_.as<U>() : nullptr, xc_.as<double>(), mask(k, n), partials_.as<double>(),
                                          sums_.as<double>() + k * total_sums_ + sum_off_[n], err_.as<int>(), s,
                                          moments);
                    });
@@ -1488,8 +1453,6 @@ class EngineImpl final : public Engine {
         build_mean_var(cot_dev_.as<double>(), np, B, K_, counts_dev_.as<double>(), levels_, i_mean_, i_var_,
                        mv_.as<double>(), s);
       });
-    if (gBrc_.p)  // level 0's products VJP beside the coarser levels
-      fork(0, [&] { typed(0, [&](auto t) { reverse_products<typename decltype(t)::type>(0); }); });
     for (int n = levels_ - 1; n >= 0; --n)
       typed(n, [&](auto t) { reverse_level<typename decltype(t)::type>(n); });
     for (int k = 0; k < launch_sets() && !opt_.cross; ++k)  // the cross plan has no mean or variance
@@ -1500,32 +1463,6 @@ class EngineImpl final : public Engine {
                            npix(0), gX_[0].as<U>(), s, segmented() ? seg_dev_[0].as<i64>() : nullptr, K_);
         });
       });
-  }
-
-  // the products VJP of level n: the cotangents of z and of the branches
-  template <typename U>
-  void reverse_products(int n) {
-    const int L = opt_.L, B = opt_.B;
-    cudaStream_t s = stream_;
-    const i64 N = npix(n);
-    const ProductShape& sh = shapes_[n];
-    // cotangent matrices and S1 scales in the field precision, one set per
-    // mask, staged for every level before the sweep; the products VJP of
-    // mask k > 0 adds to that of the masks before it
-    const double sz = sizeof(U);
-    for (int k = 0; k < launch_sets(); ++k) {
-      const U* Mdev = reinterpret_cast<const U*>(stage_dev_.as<unsigned char>() + stage_m_[(size_t)n * K_ + k]);
-      const U* sdev = reinterpret_cast<const U*>(stage_dev_.as<unsigned char>() + stage_s_[(size_t)n * K_ + k]);
-      prof_.launch(Profiler::PROD_REV, 1, (double)B * L * N * sh.K * 4 * sz, (double)B * L * N * sh.K * sh.K * 8.0,
-                   s, [&] {
-                     if (opt_.cross)
-                       cross_reverse<U>(sh.K, N, B, zf<U>(n), brf<U>(n), Mdev, sdev, mask(k, n), k > 0,
-                                        gzf<U>(n), gbrf<U>(n), s);
-                     else
-                       products_reverse<U>(sh, zf<U>(n), brf<U>(n), Mdev, sdev, mask(k, n), k > 0,
-                                           gzf<U>(n), gbrf<U>(n), s);
-                   });
-    }
   }
 
   // one level of the reverse sweep (field type U); M: the level's cotangent
@@ -1558,20 +1495,34 @@ class EngineImpl final : public Engine {
                         xc_.as<double>() + (size_t)n * B, tile(n, T_FWD_Z));
       });
       prof_.launch(Profiler::ELEM, 1, 16.0 * B * L, 0.0, s,
-                   [&] { branch_constants(zc_.as<double>(), n, B, L, rc(n), s); });
+                   [&] { branch_constants(zc_.as<double>(), n, B, L, rc_.as<double>(), s); });
       prof_.launch(Profiler::CONV_FWD, 1, conv_bytes(op, Rb, true, false), conv_flops(op, Rb), s, [&] {
-        conv_forward<U>(op, Mod_[n].as<U>(), Rb, brf<U>(n), nullptr, 0, 0, 0, s, err_.as<int>(), rc(n),
+        conv_forward<U>(op, Mod_[n].as<U>(), Rb, brf<U>(n), nullptr, 0, 0, 0, s, err_.as<int>(), rc_.as<double>(),
                         tile(n, T_FWD_BR));
       });
     }
+    // cotangent matrices and S1 scales in the field precision, one set per
+    // mask, staged for every level before the sweep; the products VJP of
+    // mask k > 0 adds to that of the masks before it
     const double sz = sizeof(U);
-    if (n == 0 && gBrc_.p) join();
-    else reverse_products<U>(n);
+    for (int k = 0; k < launch_sets(); ++k) {
+      const U* Mdev = reinterpret_cast<const U*>(stage_dev_.as<unsigned char>() + stage_m_[(size_t)n * K_ + k]);
+      const U* sdev = reinterpret_cast<const U*>(stage_dev_.as<unsigned char>() + stage_s_[(size_t)n * K_ + k]);
+      prof_.launch(Profiler::PROD_REV, 1, (double)B * L * N * sh.K * 4 * sz, (double)B * L * N * sh.K * sh.K * 8.0,
+                   s, [&] {
+                     if (opt_.cross)
+                       cross_reverse<U>(sh.K, N, B, zf<U>(n), brf<U>(n), Mdev, sdev, mask(k, n), k > 0,
+                                        gZ_.as<U>(), gBr_.as<U>(), s);
+                     else
+                       products_reverse<U>(sh, zf<U>(n), brf<U>(n), Mdev, sdev, mask(k, n), k > 0,
+                                           gZ_.as<U>(), gBr_.as<U>(), s);
+                   });
+    }
     const int R = B * (n + 1) * L;
     prof_.launch(Profiler::CONV_ADJ, adjoint_tiles_usable(op, sizeof(U), R, adj_ptr()) ? 2 : 1,
                  conv_bytes(op, R, false, true), conv_flops(op, R), s,
                  [&] {
-                   conv_adjoint<U>(op, gbrf<U>(n), R, gmod, true, s, adj_ptr(), err_.as<int>(), nullptr,
+                   conv_adjoint<U>(op, gBr_.as<U>(), R, gmod, true, s, adj_ptr(), err_.as<int>(), nullptr,
                                    tile(n, T_ADJ_BR));
                  });
     // the modulus VJP of z (gZ += gmod z / |z|): inside the coloured adjoint
@@ -1584,11 +1535,11 @@ class EngineImpl final : public Engine {
     const bool fuse = conv_adjoint_fuses_modulus(op, sizeof(U), B, adj_ptr(), err_.as<int>());
     if (!fuse)
       prof_.launch(Profiler::ELEM, 1, (double)B * L * N * 5 * sz, (double)B * L * N * 6.0, s, [&] {
-        modulus_vjp_add<U>(zf<U>(n), gmod + n * L, B * (n + 1) * L, (n + 1) * L, gzf<U>(n), N, B, L, s);
+        modulus_vjp_add<U>(zf<U>(n), gmod + n * L, B * (n + 1) * L, (n + 1) * L, gZ_.as<U>(), N, B, L, s);
       });
     prof_.launch(Profiler::CONV_ADJ, adjoint_tiles_usable(op, sizeof(U), B, adj_ptr()) ? 2 : 1,
                  conv_bytes(op, B, false, false), conv_flops(op, B), s, [&] {
-                   conv_adjoint<U>(op, gzf<U>(n), B, gX_[n].as<U>(), false, s, adj_ptr(), err_.as<int>(),
+                   conv_adjoint<U>(op, gZ_.as<U>(), B, gX_[n].as<U>(), false, s, adj_ptr(), err_.as<int>(),
                                    fuse ? &madd : nullptr, tile(n, T_ADJ_Z));
                  });
     if (n + 1 < levels_ && !levels_given_)  // maps given per level: no chain through the decimation
@@ -1787,62 +1738,6 @@ class EngineImpl final : public Engine {
     }
     STL_CUDA(cudaGraphLaunch(g.exec, stream_));
   }
-
-  // Branches of a sweep that depend on less than the launches before them go
-  // to streams of their own (captured as parallel branches of the sweep's
-  // graph), so that the short kernels of the coarse levels run beside the long
-  // ones of the fine: fork(i, f) runs f after the work queued so far, on side
-  // stream i; join() makes the sweep's stream wait for every side stream used.
-  // One stream where the sweeps run kernel by kernel ("graphs": false,
-  // profiling) and where levels share buffers (recomputed fields).
-  std::vector<cudaStream_t> side_;
-  std::vector<cudaEvent_t> side_ev_;  // per side stream, then one for the forks
-  std::vector<char> side_used_;
-  bool forks() const { return opt_.graphs && !recompute_; }
-  template <typename F>
-  void fork(int i, F&& f) {
-    if (!forks() || prof_.on) {
-      f();
-      return;
-    }
-    if (side_.empty()) {
-      for (int k = 0; k <= levels_; ++k) {
-        cudaEvent_t e;
-        STL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        side_ev_.push_back(e);
-        if (k == levels_) break;
-        cudaStream_t st;
-        STL_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        side_.push_back(st);
-      }
-      side_used_.assign(levels_, 0);
-    }
-    cudaStream_t main = stream_;
-    STL_CUDA(cudaEventRecord(side_ev_[levels_], main));
-    STL_CUDA(cudaStreamWaitEvent(side_[i], side_ev_[levels_], 0));
-    side_used_[i] = 1;
-    stream_ = side_[i];
-    try {
-      f();
-    } catch (...) {
-      stream_ = main;
-      throw;
-    }
-    stream_ = main;
-  }
-  void join() {
-    for (size_t i = 0; i < side_used_.size(); ++i)
-      if (side_used_[i]) {
-        STL_CUDA(cudaEventRecord(side_ev_[i], side_[i]));
-        STL_CUDA(cudaStreamWaitEvent(stream_, side_ev_[i], 0));
-        side_used_[i] = 0;
-      }
-  }
-  std::vector<size_t> part_off_;  // partial sums of every level (doubles)
-  DevMem gZc_, gBrc_;             // cotangents of the levels above 0, or none
-  template <typename U> U* gzf(int n) { return n > 0 && gZc_.p ? gZc_.as<U>() : gZ_.as<U>(); }
-  template <typename U> U* gbrf(int n) { return n > 0 && gBrc_.p ? gBrc_.as<U>() : gBr_.as<U>(); }
-  double* rc(int n) { return rc_.as<double>() + (size_t)n * opt_.B * levels_ * opt_.L; }
 
   // recompute field store: the one z and branch buffer of every level
   bool recompute_ = false;
