@@ -19,6 +19,7 @@
 #include <cstdio>
 
 #include "engine.cuh"
+#include "stages.cuh"
 
 namespace stl {
 
@@ -58,7 +59,6 @@ __device__ __forceinline__ i64 rot_cell(i64 c, int k, int o2) {
 // the CTA's shared memory when it exited).  Either way the launch's results
 // are discarded by the host.
 constexpr int kWaitLimit = 1 << 20;
-constexpr int kErrWait = 1, kErrDrain = 2;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -92,6 +92,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned phase) {
   }
   return false;
 }
+// the stage protocol's barriers (StageStream)
+struct StageBarriers {
+  static __device__ __forceinline__ void init(uint64_t* bar, unsigned count) { mbar_init(bar, count); }
+  static __device__ __forceinline__ void init_done() {
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  static __device__ __forceinline__ bool wait(uint64_t* bar, unsigned phase) { return mbar_wait(bar, phase); }
+  static __device__ __forceinline__ void arrive(uint64_t* bar) { mbar_arrive(bar); }
+  static __device__ __forceinline__ void sync() { __syncwarp(); }
+  static __device__ __forceinline__ bool all(bool ok) { return __all_sync(0xffffffffu, ok); }
+};
 
 // BYTES (4, 8 or 16) global -> shared, zero fill when !live, not waited
 template <int BYTES>
@@ -426,15 +438,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_conv_fwd_tiles(
   const int S4 = ((S + 3) / 4) * 4;  // slots per tile in the tile-major index table
   S = tile_slots[tile];              // the tile's rows use no later slot
   const int nch = (S + SC - 1) / SC;
+  StageStream<StageBarriers, NST, 0, kFwdThreads / 32> cs(bar, empty);
+  cs.nch = nch;
   if (tid == 0) {
-#pragma unroll
-    for (int q = 0; q < NST; ++q) {
-      mbar_init(&bar[q], 1);
-      mbar_init(&empty[q], kFwdThreads / 32);
-    }
+    cs.init();
     fail = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
   auto issue = [&](int c) {
@@ -449,8 +457,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_conv_fwd_tiles(
       bulk_g2s(base + (size_t)sl * kAdjTile * 8 * sizeof(T), coef + ((i64)(s0 + sl) * n_rep + u0) * 8, cb, &bar[st]);
     bulk_g2s(base + kStageCoef, lcell_t + ((i64)tile * S4 + s0) * kAdjTile, lb, &bar[st]);
   };
-  if (tid == 0)
-    for (int c = 0; c < min(nch, NST); ++c) issue(c);
+  if (tid == 0) cs.begin(nch, issue);
   const int32_t* tc = tile_cells + (i64)tile * kAdjCells;
   // planes of pc >= nc + 1 cells, pc chosen so that consecutive planes start
   // 32 bytes apart modulo 128: the 4 rotations of a row, which read the same
@@ -470,22 +477,12 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_conv_fwd_tiles(
     for (int j = 0; j < 8; ++j) acc[rb][j] = (T)0;
   const T* sxk = sx + (size_t)k * pc * RB;
   __syncthreads();  // the cell gather, before any thread reads it
-  // The chunks: every warp waits for a stage's copies on its own, reads it,
-  // then releases it (one arrival per warp on `empty`); thread 0 refills a
-  // stage once every warp has released it.  No CTA-wide barrier in the loop:
-  // warps drift apart by up to a stage.
-  const int lane = tid & 31;
-  bool ok = true;
-  int issued = min(nch, NST);  // chunks issued (thread 0's count)
+  // The chunks: no CTA-wide barrier in the loop, warps drift apart by up to a
+  // stage (StageStream; a stage is refilled as soon as every warp released it).
   for (int c = 0; c < nch; ++c) {
-    const int st = c % NST;
-    const unsigned par = (unsigned)(c / NST) & 1;
-    if (!mbar_wait(&bar[st], par)) {
-      ok = false;
-      break;
-    }
-    const unsigned char* base = smem_raw + st * kStage;
-    const T* cs = reinterpret_cast<const T*>(base);
+    if (!cs.wait(c)) break;
+    const unsigned char* base = smem_raw + (c % NST) * kStage;
+    const T* cf = reinterpret_cast<const T*>(base);
     const uint16_t* ls = reinterpret_cast<const uint16_t*>(base + kStageCoef);
     const int sn = min(SC, S - c * SC);
     if (row < rows) {
@@ -493,32 +490,19 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_conv_fwd_tiles(
       for (int sl = 0; sl < SC; ++sl) {
         if (sl < sn) {
           T w[8];
-          load8_shared(cs + ((size_t)sl * kAdjTile + row) * 8, w);
+          load8_shared(cf + ((size_t)sl * kAdjTile + row) * 8, w);
           T xv[RB];
           loadR_shared<RB>(sxk + (size_t)ls[sl * kAdjTile + row] * RB, xv);
           fma_rows<RB>(acc, w, xv);
         }
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[st]);
-    if (tid == 0 && c + NST < nch) {
-      if (!mbar_wait(&empty[st], par)) {
-        ok = false;
-        break;
-      }
-      issue(c + NST);
-      issued = c + NST + 1;
-    }
+    cs.release(c, tid, issue);
   }
-  if (!ok) fail = 1;
+  if (!cs.ok) fail = 1;
   __syncthreads();
-  if (fail) {  // thread 0 waits (bounded) for the copies it may have in flight
-    if (tid == 0) {
-      bool drained = true;
-      for (int q = max(0, issued - NST); q < issued; ++q) drained &= mbar_wait(&bar[q % NST], (q / NST) & 1);
-      atomicMax(err, drained ? kErrWait : kErrDrain);
-    }
+  if (fail) {
+    if (tid == 0) atomicMax(err, cs.drain());
     return;
   }
   if (row >= rows) return;
@@ -940,52 +924,33 @@ constexpr size_t kGridStageBytes = 8192;
 __device__ __forceinline__ int grid_x(int ul) { return (ul & 1) | ((ul >> 1) & 2) | ((ul >> 2) & 4); }
 __device__ __forceinline__ int grid_y(int ul) { return grid_x(ul >> 1); }
 
-// The coefficient stream of a CTA: stage c % kGridStages holds the slots
-// c SC .. of the tile.  Thread 0 fills a stage by one bulk copy; every warp
-// waits for it on its own and releases it with one arrival; a stage is
-// refilled a chunk after it was released, so the refill seldom waits.  Every
-// wait is bounded.
+// The coefficient stream of a CTA (StageStream): stage c % kGridStages holds the
+// slots c SC .. of the tile, filled by one bulk copy.
 template <typename T, int WARPS>
-struct GridStream {
+struct GridStream : StageStream<StageBarriers, kGridStages, 1, WARPS> {
+  typedef StageStream<StageBarriers, kGridStages, 1, WARPS> Base;
   static constexpr int SC = grid_sc<T>();
   static_assert(SC * kGridSlot * sizeof(T) == kGridStageBytes && kGridPad % SC == 0, "whole stages");
   unsigned char* base;
-  uint64_t *full, *empty;
   const T* src;  // the tile's first coefficient
-  int S, nch, issued;
-  __device__ __forceinline__ void init() {  // thread 0
-    for (int q = 0; q < kGridStages; ++q) {
-      mbar_init(&full[q], 1);
-      mbar_init(&empty[q], WARPS);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  // slots of the tile: whole stages (kGridPad)
+  __device__ __forceinline__ GridStream(unsigned char* stages, uint64_t* bar, const T* first, int slots)
+      : Base(bar, bar + kGridStages), base(stages), src(first) {
+    this->nch = slots / SC;
   }
   __device__ __forceinline__ void issue(int c) {  // thread 0
     const int st = c % kGridStages;
-    mbar_expect_tx(&full[st], kGridStageBytes);
-    bulk_g2s(base + st * kGridStageBytes, src + (i64)c * SC * kGridSlot, kGridStageBytes, &full[st]);
-    issued = c + 1;
+    mbar_expect_tx(&this->full[st], kGridStageBytes);
+    bulk_g2s(base + st * kGridStageBytes, src + (i64)c * SC * kGridSlot, kGridStageBytes, &this->full[st]);
   }
-  __device__ __forceinline__ bool wait(int c) { return mbar_wait(&full[c % kGridStages], (c / kGridStages) & 1); }
+  __device__ __forceinline__ void begin() {
+    Base::begin(this->nch, [this](int c) { issue(c); });
+  }
   __device__ __forceinline__ const T* stage(int c) const {
     return reinterpret_cast<const T*>(base + (c % kGridStages) * kGridStageBytes);
   }
-  // after chunk c was read by the warp; thread 0 refills the stage of chunk c - 1
-  __device__ __forceinline__ bool release(int c, int tid) {
-    __syncwarp();
-    if ((tid & 31) == 0) mbar_arrive(&empty[c % kGridStages]);
-    if (tid == 0 && c > 0 && c - 1 + kGridStages < nch) {
-      if (!mbar_wait(&empty[(c - 1) % kGridStages], ((c - 1) / kGridStages) & 1)) return false;
-      issue(c - 1 + kGridStages);
-    }
-    return true;
-  }
-  // thread 0, after a failed wait anywhere: the copies in flight land (bounded)
-  __device__ __forceinline__ int drain() {
-    bool ok = true;
-    for (int q = max(0, issued - kGridStages); q < issued; ++q) ok &= wait(q);
-    return ok ? kErrWait : kErrDrain;
+  __device__ __forceinline__ void release(int c, int tid) {
+    Base::release(c, tid, [this](int q) { issue(q); });
   }
 };
 
@@ -1171,14 +1136,8 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) 
   T rs[8];
   load8(rowsum + u * 8, rs);
   const i64 s0 = start[tile];
-  GridStream<T, NT / 32> cs;
-  cs.base = smem_raw;
-  cs.full = bar;
-  cs.empty = bar + kGridStages;
-  cs.src = coef + s0 * kGridSlot;
-  cs.S = (int)(start[tile + 1] - s0);
-  cs.nch = cs.S / SC;  // a tile's slots are whole stages
-  cs.issued = 0;
+  const int S = (int)(start[tile + 1] - s0);
+  GridStream<T, NT / 32> cs(smem_raw, bar, coef + s0 * kGridSlot, S);
   // the tile's cells, 4 rotations x RB rows a group; positions no row reads: zero
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
@@ -1194,9 +1153,9 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) 
   if (tid == 0) {
     cs.init();
     fail = 0;
-    for (int c = 0; c < min(cs.nch, kGridStages); ++c) cs.issue(c);
+    cs.begin();
   }
-  for (int i = tid; i < cs.S; i += NT) soff[i] = off[s0 + i] * RB;
+  for (int i = tid; i < S; i += NT) soff[i] = off[s0 + i] * RB;
   // the sums start from the rows' constants times the row sums of the coefficients
   GridRows<T, RB> acc[4][8];
 #pragma unroll
@@ -1210,12 +1169,8 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) 
   const T* px = planes + (size_t)fg * kPlanes + ((grid_y(row) + kGridHalo) * kGridP + grid_x(row) + kGridHalo) * RB;
   cp_async_wait_all();
   __syncthreads();
-  bool ok = true;
   for (int c = 0; c < cs.nch; ++c) {
-    if (!cs.wait(c)) {
-      ok = false;
-      break;
-    }
+    if (!cs.wait(c)) break;
     const T* cf = cs.stage(c) + row * VL;
 #pragma unroll
     for (int sl = 0; sl < SC; ++sl) {
@@ -1233,12 +1188,9 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) 
         for (int k = 0; k < 4; ++k) gr_fma(acc[k][j], wj, xv[k]);
       }
     }
-    if (!cs.release(c, tid)) {
-      ok = false;
-      break;
-    }
+    cs.release(c, tid);
   }
-  if (!ok) fail = 1;
+  if (!cs.ok) fail = 1;
   __syncthreads();
   if (fail) {
     if (tid == 0) atomicMax(err, cs.drain());
@@ -1318,20 +1270,14 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_adj_ctas<T, RB, FG>())) 
     }
   }
   const i64 s0 = start[tile];
-  GridStream<T, NT / 32> cs;
-  cs.base = smem_raw;
-  cs.full = bar;
-  cs.empty = bar + kGridStages;
-  cs.src = coef + s0 * kGridSlot;
-  cs.S = (int)(start[tile + 1] - s0);
-  cs.nch = cs.S / SC;  // a tile's slots are whole stages
-  cs.issued = 0;
+  const int S = (int)(start[tile + 1] - s0);
+  GridStream<T, NT / 32> cs(smem_raw, bar, coef + s0 * kGridSlot, S);
   if (tid == 0) {
     cs.init();
     fail = 0;
-    for (int c = 0; c < min(cs.nch, kGridStages); ++c) cs.issue(c);
+    cs.begin();
   }
-  for (int i = tid; i < cs.S; i += NT) soff[i] = off[s0 + i] * RB;
+  for (int i = tid; i < S; i += NT) soff[i] = off[s0 + i] * RB;
   // the combine's positions of this thread's tile cells
   const int nc = tile_nc[tile];
   constexpr int NL = (kGridCells * FG + NT - 1) / NT;
@@ -1381,12 +1327,8 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_adj_ctas<T, RB, FG>())) 
   for (int i = lane; i < kBox / VL; i += 32) reinterpret_cast<uint4*>(box)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
   T* sum = box + ((grid_y(lane) + kGridHalo) * kGridP + grid_x(lane) + kGridHalo) * RB;
-  bool ok = true;
   for (int c = 0; c < cs.nch; ++c) {
-    if (!cs.wait(c)) {
-      ok = false;
-      break;
-    }
+    if (!cs.wait(c)) break;
     const T* cf = cs.stage(c) + row * VL;
     T w[8];
     grid_coef(cf, w);
@@ -1417,12 +1359,9 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_adj_ctas<T, RB, FG>())) 
 #pragma unroll
         for (int q = 0; q < 8; ++q) w[q] = wn[q];
     }
-    if (!cs.release(c, tid)) {
-      ok = false;
-      break;
-    }
+    cs.release(c, tid);
   }
-  if (!ok) fail = 1;
+  if (!cs.ok) fail = 1;
   __syncthreads();
   if (fail) {
     if (tid == 0) atomicMax(err, cs.drain());

@@ -1,0 +1,79 @@
+// The staged coefficient stream of the tiled wavelets: the chunks of a CTA pass
+// through STAGES stages of shared memory, chunk c through stage c % STAGES.
+// Thread 0 fills the stages by bulk asynchronous copies; every warp waits for a
+// stage on its own, reads it and releases it with one arrival; thread 0 refills
+// the stage of chunk c - LAG after it released chunk c (LAG 1: the other warps have had a
+// chunk's time to release it, so the refill seldom waits).
+//
+// Every wait is bounded, and a warp leaves the chunks as a whole: a wait that ran
+// out in any lane, or thread 0's wait for a stage to be free, is seen by all lanes
+// of the warp at their next wait() (one vote a chunk).  Lanes that left alone
+// would wait at the CTA's barrier while the rest of their warp waits for them at the
+// next __syncwarp.  The warps of a CTA that wait for a chunk which is never
+// issued run out by themselves, so all reach the CTA's barrier.
+//
+// P supplies the mbarriers and the warp's barrier and vote: the device's in
+// kernels.cu, threads that check for lanes left behind in the host test.
+#pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define STL_STAGE_FN __device__ __forceinline__
+#else
+#define STL_STAGE_FN inline
+#endif
+
+namespace stl {
+
+// error flag of a launch: a wait ran out and the copies in flight then landed, or
+// they did not
+constexpr int kErrWait = 1, kErrDrain = 2;
+
+template <class P, int STAGES, int LAG, int WARPS>
+struct StageStream {
+  uint64_t *full, *empty;  // [STAGES]: a stage's copies have landed; every warp has read it
+  int nch = 0;             // chunks
+  int issued = 0;          // chunks issued (thread 0)
+  bool ok = true;          // no wait of this thread (after wait(): of its warp) ran out
+  STL_STAGE_FN StageStream(uint64_t* f, uint64_t* e) : full(f), empty(e) {}
+  STL_STAGE_FN void init() {  // thread 0, before the first issue and the CTA's barrier
+    for (int q = 0; q < STAGES; ++q) {
+      P::init(&full[q], 1);
+      P::init(&empty[q], WARPS);
+    }
+    P::init_done();
+  }
+  // thread 0: issue(c) queues the copies of chunk c into its stage
+  template <class F>
+  STL_STAGE_FN void begin(int chunks, F&& issue) {
+    for (; issued < chunks && issued < STAGES; ++issued) issue(issued);
+  }
+  // chunk c has landed; false in every lane of the warp when a wait ran out
+  STL_STAGE_FN bool wait(int c) {
+    ok = ok && P::wait(&full[c % STAGES], (unsigned)(c / STAGES) & 1);
+    return ok = P::all(ok);
+  }
+  // after the warp read chunk c
+  template <class F>
+  STL_STAGE_FN void release(int c, int tid, F&& issue) {
+    P::sync();
+    if ((tid & 31) == 0) P::arrive(&empty[c % STAGES]);
+    const int d = c - LAG;
+    if (tid == 0 && d >= 0 && d + STAGES < nch) {
+      ok = P::wait(&empty[d % STAGES], (unsigned)(d / STAGES) & 1);
+      if (ok) {
+        issue(d + STAGES);
+        issued = d + STAGES + 1;
+      }
+    }
+  }
+  // thread 0, after a wait ran out anywhere: the copies in flight land (bounded)
+  STL_STAGE_FN int drain() {
+    bool landed = true;
+    for (int q = issued > STAGES ? issued - STAGES : 0; q < issued; ++q)
+      landed &= P::wait(&full[q % STAGES], (unsigned)(q / STAGES) & 1);
+    return landed ? kErrWait : kErrDrain;
+  }
+};
+
+}  // namespace stl
