@@ -92,6 +92,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned phase) {
   }
   return false;
 }
+// Between a thread's reads of a stage of shared memory and the barrier after which
+// the copy engine (the async proxy) writes the stage again: without the fence the
+// barrier does not order the two.
+__device__ __forceinline__ void stage_reads_done() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // the stage protocol's barriers (StageStream)
 struct StageBarriers {
   static __device__ __forceinline__ void init(uint64_t* bar, unsigned count) { mbar_init(bar, count); }
@@ -101,6 +105,7 @@ struct StageBarriers {
   }
   static __device__ __forceinline__ bool wait(uint64_t* bar, unsigned phase) { return mbar_wait(bar, phase); }
   static __device__ __forceinline__ void arrive(uint64_t* bar) { mbar_arrive(bar); }
+  static __device__ __forceinline__ void reads_done() { stage_reads_done(); }
   static __device__ __forceinline__ void sync() { __syncwarp(); }
   static __device__ __forceinline__ bool all(bool ok) { return __all_sync(0xffffffffu, ok); }
 };
@@ -876,8 +881,10 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
         dot8_rows<RB>(w, g, a);
         addR_shared<RB>(acc + ((size_t)lc * 4 + k) * RB, a);
       }
-      __syncthreads();  // the slot's sums are in: the next slot may read them
+      if (sl + 1 < sn) __syncthreads();  // the slot's sums are in: the next slot may read them
     }
+    stage_reads_done();
+    __syncthreads();
     if (tid == 0 && c + 2 < nch) issue(c + 2);
   }
   if (fail) {
@@ -1620,6 +1627,7 @@ __global__ void __launch_bounds__(kMmaFwdThreads, 2) k_conv_fwd_mma(
         for (int q = 0; q < 4; ++q) acc[i][mt][q] += d[q];
       }
     }
+    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
     if (tid == 0 && c + NS < nch) issue(c + NS);
   }
@@ -1781,6 +1789,7 @@ __global__ void __launch_bounds__(kMmaAdjThreads, 2) k_conv_adj_mma(
         *s1 = v1;
       }
     }
+    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
     if (tid == 0 && c + NS < nch) issue(c + NS);
   }
@@ -2076,6 +2085,7 @@ __global__ void __launch_bounds__(kProdMaxWarps * 32, 1) k_products(
         f[i] = (T)0;
       }
     }
+    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
     if (threadIdx.x == 0 && c + kProdStages < nchunks) issue(c + kProdStages);
   }

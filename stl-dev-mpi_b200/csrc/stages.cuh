@@ -12,7 +12,11 @@
 // next __syncwarp.  The warps of a CTA that wait for a chunk which is never
 // issued run out by themselves, so all reach the CTA's barrier.
 //
-// P supplies the mbarriers and the warp's barrier and vote: the device's in
+// The stages are read by ordinary loads and written by the copy engine, another
+// proxy: the barriers order the two only together with a proxy fence, which every
+// lane executes between its reads of a stage and the release.
+//
+// P supplies the mbarriers, the fence and the warp's barrier and vote: the device's in
 // kernels.cu, threads that check for lanes left behind in the host test.
 #pragma once
 #include <cstdint>
@@ -56,6 +60,7 @@ struct StageStream {
   // after the warp read chunk c
   template <class F>
   STL_STAGE_FN void release(int c, int tid, F&& issue) {
+    P::reads_done();
     P::sync();
     if ((tid & 31) == 0) P::arrive(&empty[c % STAGES]);
     const int d = c - LAG;

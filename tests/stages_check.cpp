@@ -1,7 +1,8 @@
 // The staged stream of the tiled wavelets (csrc/stages.cuh) run by host threads,
 // one a lane, with mbarriers, votes and barriers of their own: a wait that runs
 // out, in thread 0's refill or in one lane, must leave no lane waiting for another
-// for good, and every copy issued must have landed at the end.  Exits
+// for good, and every copy issued must have landed at the end; no copy may be
+// issued into a stage that a lane has read without a proxy fence since.  Exits
 // nonzero on a failure.
 #include "stages.cuh"
 
@@ -60,6 +61,7 @@ struct Meet {  // a barrier of n threads with the conjunction of their votes
 Meet warp_meet[kWarps], cta_meet;
 
 thread_local int tid;
+unsigned unfenced[kLanes];  // the stages a lane has read since its last fence
 std::function<bool(uint64_t*, unsigned)> runs_out;  // the wait of this thread that is made to fail
 
 struct Sim {
@@ -73,6 +75,10 @@ struct Sim {
   static void arrive(uint64_t* bar) {
     std::lock_guard<std::mutex> g(mu);
     arrive_locked(bars[bar]);
+  }
+  static void reads_done() {
+    std::lock_guard<std::mutex> g(mu);
+    unfenced[tid] = 0;
   }
   static void sync() { warp_meet[tid / 32](true); }
   static bool all(bool ok) { return warp_meet[tid / 32](ok); }
@@ -103,7 +109,8 @@ void engine() {
 template <int STAGES, int LAG>
 int run(int nch, int which) {
   uint64_t bar[2 * STAGES];
-  int stage[STAGES], fail = 0, err = 0, hung = 0, wrong = 0, in_flight = 0;
+  int stage[STAGES], fail = 0, err = 0, hung = 0, wrong = 0, in_flight = 0, unordered = 0;
+  for (unsigned& u : unfenced) u = 0;
   for (int& v : stage) v = -1;
   bars.clear();
   for (Meet& m : warp_meet) m = Meet{32};
@@ -127,6 +134,7 @@ int run(int nch, int which) {
         cs.nch = nch;
         auto issue = [&](int c) {
           std::lock_guard<std::mutex> g(mu);
+          for (unsigned u : unfenced) unordered += u >> (c % STAGES) & 1;
           copies.push_back({&bar[c % STAGES], &stage[c % STAGES], c});
           cv.notify_all();
         };
@@ -140,6 +148,7 @@ int run(int nch, int which) {
           {
             std::lock_guard<std::mutex> g(mu);
             wrong += stage[c % STAGES] != c;
+            unfenced[tid] |= 1u << (c % STAGES);
           }
           Sim::sync();  // the slots of the adjoint
           cs.release(c, tid, issue);
@@ -166,10 +175,11 @@ int run(int nch, int which) {
   }
   eng.join();
   const int want = which && nch > STAGES + LAG ? stl::kErrWait : 0;
-  const bool good = !hung && !wrong && !in_flight && err == want && (want ? fired : !fail);
+  const bool good = !hung && !wrong && !in_flight && !unordered && err == want && (want ? fired : !fail);
   if (!good)
-    std::printf("stages %d lag %d chunks %d case %d: %d lanes left waiting, %d wrong reads, %d copies in flight, error %d (%d)\n",
-                STAGES, LAG, nch, which, hung, wrong, in_flight, err, want);
+    std::printf("stages %d lag %d chunks %d case %d: %d lanes left waiting, %d wrong reads, %d copies in flight, "
+                "%d reads not ordered before a copy, error %d (%d)\n",
+                STAGES, LAG, nch, which, hung, wrong, in_flight, unordered, err, want);
   return !good;
 }
 

@@ -1,6 +1,7 @@
 """The staged coefficient stream of the tiled wavelets (csrc/stages.cuh) on host
 threads: a bounded wait that runs out leaves no lane of a warp waiting for the
-others, and the copies in flight land first (a C++ check compiled here)."""
+others, the copies in flight land first, and a stage's reads are fenced before the
+copy engine writes it again (a C++ check compiled here)."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -10,7 +11,7 @@ import pytest
 ROOT = Path(__file__).resolve().parents[1]
 
 
-def test_waits_that_run_out_leave_no_lane_behind(tmp_path):
+def test_staged_stream_on_host_threads(tmp_path):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no host C++ compiler")
