@@ -252,7 +252,11 @@ char* stlp_info(StlpHandle* h) {
     for (size_t i = 0; i < ol.size(); ++i)
       js << (i ? ", " : "") << "{\"slots\": " << ol[i][0] << ", \"tile_cells\": " << ol[i][1]
          << ", \"coloured\": " << (ol[i][2] == 1 || ol[i][2] == 2 ? "true" : "false") << ", \"layout\": \""
-         << (ol[i][2] == 3 ? "tensor_cores" : ol[i][2] == 2 ? "tensor_cores+coloured" : ol[i][2] == 1 ? "coloured" : "rows")
+         << (ol[i][2] == 4   ? "grid"
+             : ol[i][2] == 3 ? "tensor_cores"
+             : ol[i][2] == 2 ? "tensor_cores+coloured"
+             : ol[i][2] == 1 ? "coloured"
+                             : "rows")
          << "\", \"warp_cells\": "
          << ol[i][3] << "}";
     js << "], \"tile_heights\": [";

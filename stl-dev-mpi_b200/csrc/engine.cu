@@ -1301,7 +1301,7 @@ class EngineImpl final : public Engine {
     std::vector<std::array<int, 4>> v;
     for (const auto& c : conv_)
       v.push_back({c.mma ? c.m_S : c.S, c.mma ? c.m_pc : c.max_tile_cells,
-                   c.mma_adj ? 3 : c.mma ? 2 : c.colored || c.grid ? 1 : 0, c.mma_adj ? c.m_wl : 0});
+                   c.grid ? 4 : c.mma_adj ? 3 : c.mma ? 2 : c.colored ? 1 : 0, c.mma_adj ? c.m_wl : 0});
     return v;
   }
 

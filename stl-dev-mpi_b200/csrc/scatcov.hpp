@@ -194,7 +194,9 @@ class Engine {
   virtual bool profiling() const = 0;
   // Mean cells read per row of each level's wavelet operator.
   virtual std::vector<double> mean_slots() const = 0;
-  // Per level: slots per stored row, most cells of a tile, coloured layout (0/1).
+  // Per level: slots per stored row (grid: most of a tile), most cells of a tile, the
+  // layout (0 per-row slots, 1 coloured, 2 tensor cores with the coloured adjoint, 3
+  // tensor cores, 4 grid), most cells of a warp (3).
   virtual std::vector<std::array<int, 4>> operator_layout() const = 0;
   virtual bool recomputes() const = 0;  // the field store in use (after prepare)
   virtual size_t kept_field_bytes() const = 0;  // bytes of z and branches of every level (after prepare)

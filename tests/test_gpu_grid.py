@@ -2,7 +2,8 @@
 statistics and their gradient against the FP64 oracle where the layout can go
 wrong -- nside 16, every tile of which reaches across face edges and vertices
 (displacements of 5 cells), the first FP32 level above nside 32, and batches whose
-row counts give a CTA one or two groups of 1, 2 or 4 rows."""
+row counts give a CTA one or two groups of 1, 2 or 4 rows.  Each level is in the
+layout its size calls for."""
 import numpy as np
 import pytest
 
@@ -21,6 +22,8 @@ def test_grid_wavelets_match_the_oracle(nside, J, batch, dtype):
     e = stl_b200.NativeEngine(nside, J, batch=batch, dtype=dtype)
     o = O.OracleEngine(nside, J, batch=batch)
     v, r = e.forward(x)[0], o.forward(x)
+    for d, op in enumerate(e.info()["operators"]):  # not the layout that a level falls back to
+        assert op["layout"] == ("grid" if nside >> d >= 16 else "coloured"), (d, op)
     # FP64: sums of 44 products in another order; FP32: the 1e-6 criterion of the
     # statistics relative to the largest of their family, and for a gradient
     # value two chains of at most 44 and 8 rounded products: 52 * 2^-24 = 3.1e-6 of

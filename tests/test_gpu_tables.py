@@ -5,9 +5,8 @@ dia.rs:213-238) and the fine cells of every coarse pixel's smooth
 decimation (the 2-ring coarse neighbourhood's children within the cut,
 decimation.rs:108-201, through cdshealpix's kth_neighbourhood restated in
 the oracle and pinned to the reference's neighbour fixtures), against the
-FP64 oracle as sorted sets with np.array_equal.  FP64 engines hold the
-coloured layout, FP32 engines above nside 32 the tensor-core layout: both
-are read back."""
+FP64 oracle as sorted sets with np.array_equal.  Levels of nside 16 and more
+hold the grid layout, coarser ones another: all are read back."""
 import numpy as np
 import pytest
 

@@ -1,6 +1,6 @@
 """The FP32 wavelets on the tensor cores (3xTF32 mma.sync over the
 tensor-core operator layout; engine option tensor_cores "forward" or "all")
-against the FP32 CUDA-core kernels of the coloured layout (the default) and
+against the FP32 CUDA-core kernels of the grid layout (the default) and
 the FP64 path: statistics under the 1e-6 family criterion, gradients,
 bit-reproducibility, and the layout each level gets."""
 import numpy as np
@@ -45,14 +45,14 @@ def test_layout_per_level(stl):
     """FP32 levels above nside 32 hold the tensor-core layout (for the
     forward, with the coloured one for the adjoint by default; for both with
     "all"); the FP64 coarse levels and every level with tensor_cores off
-    hold the coloured one (the default)."""
-    for mode, want in ((True, "tensor_cores+coloured"), ("all", "tensor_cores"), (False, "coloured")):
+    hold the grid layout (the default), below nside 16 the coloured one."""
+    for mode, want in ((True, "tensor_cores+coloured"), ("all", "tensor_cores"), (False, "grid")):
         e = stl.NativeEngine(128, 5, dtype="float32", tensor_cores=mode)
         e.prepare()
         layouts = [o["layout"] for o in e.info()["operators"]]
         first = 2 if mode is not False else 0
         assert all(v == want for v in layouts[:first]), (mode, layouts)
-        assert all(v == "coloured" for v in layouts[first:]), (mode, layouts)
+        assert layouts[first:] == ["grid"] * (4 - first) + ["coloured"], (mode, layouts)
         e.close()
 
 
