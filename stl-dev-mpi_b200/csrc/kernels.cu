@@ -107,7 +107,6 @@ struct StageBarriers {
   static __device__ __forceinline__ void arrive(uint64_t* bar) { mbar_arrive(bar); }
   static __device__ __forceinline__ void reads_done() { stage_reads_done(); }
   static __device__ __forceinline__ void sync() { __syncwarp(); }
-  static __device__ __forceinline__ bool all(bool ok) { return __all_sync(0xffffffffu, ok); }
 };
 
 // BYTES (4, 8 or 16) global -> shared, zero fill when !live, not waited
@@ -485,12 +484,12 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_conv_fwd_tiles(
   // The chunks: no CTA-wide barrier in the loop, warps drift apart by up to a
   // stage (StageStream; a stage is refilled as soon as every warp released it).
   for (int c = 0; c < nch; ++c) {
-    if (!cs.wait(c)) break;
+    const bool landed = cs.wait(c);  // else the stage's indices may be anything
     const unsigned char* base = smem_raw + (c % NST) * kStage;
     const T* cf = reinterpret_cast<const T*>(base);
     const uint16_t* ls = reinterpret_cast<const uint16_t*>(base + kStageCoef);
     const int sn = min(SC, S - c * SC);
-    if (row < rows) {
+    if (row < rows && landed) {
 #pragma unroll
       for (int sl = 0; sl < SC; ++sl) {
         if (sl < sn) {
@@ -913,8 +912,9 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
 // grid's pitch.  A CTA holds FG groups of RB rows over one tile, which share its
 // coefficients: they arrive once a CTA by bulk copies, in stages of grid_sc()
 // slots.  Measured on one B200 (nside 1024, J 9, B 4, FP32, a forward and its
-// VJP): forward 14.5 -> 9.6 ms, adjoint 21.4 -> 15.5 ms; FP64, nside 512, J 8, B 1: 2.80 ->
-// 2.03 and 5.02 -> 2.73 ms.  The level-0 branch forward at nside 512 keeps the FMA
+// VJP): forward 14.5 -> 9.6 ms, adjoint 21.4 -> 15.6 ms; FP64, nside 512, J 8, B 1: 2.80 ->
+// 2.05 and 5.02 -> 2.82 ms (0.05-0.15 and 0.01-0.06 ms of these are the readers' proxy
+// fences).  The level-0 branch forward at nside 512 keeps the FMA
 // pipe 57 % busy (36 % before) with three CTAs an SM of 168 registers a thread; two
 // CTAs (no spills, 255 registers) took 11 % longer.  What bounds it now is the FMA
 // pipe inside the slot loop (about 170 of 160 cycles a slot and scheduler) and
@@ -1177,7 +1177,7 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_fwd_ctas<T, RB, FG>())) 
   cp_async_wait_all();
   __syncthreads();
   for (int c = 0; c < cs.nch; ++c) {
-    if (!cs.wait(c)) break;
+    cs.wait(c);
     const T* cf = cs.stage(c) + row * VL;
 #pragma unroll
     for (int sl = 0; sl < SC; ++sl) {
@@ -1335,7 +1335,7 @@ __global__ void __launch_bounds__(kGridRows * FG, (grid_adj_ctas<T, RB, FG>())) 
   __syncwarp();
   T* sum = box + ((grid_y(lane) + kGridHalo) * kGridP + grid_x(lane) + kGridHalo) * RB;
   for (int c = 0; c < cs.nch; ++c) {
-    if (!cs.wait(c)) break;
+    cs.wait(c);
     const T* cf = cs.stage(c) + row * VL;
     T w[8];
     grid_coef(cf, w);

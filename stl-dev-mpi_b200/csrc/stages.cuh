@@ -5,18 +5,18 @@
 // the stage of chunk c - LAG after it released chunk c (LAG 1: the other warps have had a
 // chunk's time to release it, so the refill seldom waits).
 //
-// Every wait is bounded, and a warp leaves the chunks as a whole: a wait that ran
-// out in any lane, or thread 0's wait for a stage to be free, is seen by all lanes
-// of the warp at their next wait() (one vote a chunk).  Lanes that left alone
-// would wait at the CTA's barrier while the rest of their warp waits for them at the
-// next __syncwarp.  The warps of a CTA that wait for a chunk which is never
-// issued run out by themselves, so all reach the CTA's barrier.
+// Every wait is bounded, and no lane leaves the chunks early: a wait that ran out
+// (thread 0's for a free stage among them) clears the thread's ok, it waits and
+// issues no more, and goes through the remaining chunks' barriers with its
+// warp.  Lanes that left alone would wait at the CTA's barrier while the rest of
+// their warp waits for them at the next __syncwarp.  The results of such a CTA are
+// not used.  A thread that is not ok may see a stage in any state.
 //
 // The stages are read by ordinary loads and written by the copy engine, another
 // proxy: the barriers order the two only together with a proxy fence, which every
 // lane executes between its reads of a stage and the release.
 //
-// P supplies the mbarriers, the fence and the warp's barrier and vote: the device's in
+// P supplies the mbarriers, the fence and the warp's barrier: the device's in
 // kernels.cu, threads that check for lanes left behind in the host test.
 #pragma once
 #include <cstdint>
@@ -38,7 +38,7 @@ struct StageStream {
   uint64_t *full, *empty;  // [STAGES]: a stage's copies have landed; every warp has read it
   int nch = 0;             // chunks
   int issued = 0;          // chunks issued (thread 0)
-  bool ok = true;          // no wait of this thread (after wait(): of its warp) ran out
+  bool ok = true;          // no wait of this thread ran out
   STL_STAGE_FN StageStream(uint64_t* f, uint64_t* e) : full(f), empty(e) {}
   STL_STAGE_FN void init() {  // thread 0, before the first issue and the CTA's barrier
     for (int q = 0; q < STAGES; ++q) {
@@ -52,11 +52,8 @@ struct StageStream {
   STL_STAGE_FN void begin(int chunks, F&& issue) {
     for (; issued < chunks && issued < STAGES; ++issued) issue(issued);
   }
-  // chunk c has landed; false in every lane of the warp when a wait ran out
-  STL_STAGE_FN bool wait(int c) {
-    ok = ok && P::wait(&full[c % STAGES], (unsigned)(c / STAGES) & 1);
-    return ok = P::all(ok);
-  }
+  // whether chunk c has landed
+  STL_STAGE_FN bool wait(int c) { return ok = ok && P::wait(&full[c % STAGES], (unsigned)(c / STAGES) & 1); }
   // after the warp read chunk c
   template <class F>
   STL_STAGE_FN void release(int c, int tid, F&& issue) {
@@ -64,7 +61,7 @@ struct StageStream {
     P::sync();
     if ((tid & 31) == 0) P::arrive(&empty[c % STAGES]);
     const int d = c - LAG;
-    if (tid == 0 && d >= 0 && d + STAGES < nch) {
+    if (tid == 0 && ok && d >= 0 && d + STAGES < nch) {
       ok = P::wait(&empty[d % STAGES], (unsigned)(d / STAGES) & 1);
       if (ok) {
         issue(d + STAGES);

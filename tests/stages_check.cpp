@@ -1,5 +1,5 @@
 // The staged stream of the tiled wavelets (csrc/stages.cuh) run by host threads,
-// one a lane, with mbarriers, votes and barriers of their own: a wait that runs
+// one a lane, with mbarriers and barriers of their own: a wait that runs
 // out, in thread 0's refill or in one lane, must leave no lane waiting for another
 // for good, and every copy issued must have landed at the end; no copy may be
 // issued into a stage that a lane has read without a proxy fence since.  Exits
@@ -39,23 +39,18 @@ void arrive_locked(Bar& b) {
   }
 }
 
-struct Meet {  // a barrier of n threads with the conjunction of their votes
+struct Meet {  // a barrier of n threads
   int n = 0, here = 0, gen = 0;
-  bool all = true, result = true;
-  bool operator()(bool vote) {
+  void operator()() {
     std::unique_lock<std::mutex> lk(mu);
     const int g = gen;
-    all = all && vote;
     if (++here == n) {
       here = 0;
-      result = all;
-      all = true;
       ++gen;
       cv.notify_all();
-      return result;
+      return;
     }
     if (!cv.wait_for(lk, kHang, [&] { return gen != g; })) throw Left{};
-    return result;
   }
 };
 Meet warp_meet[kWarps], cta_meet;
@@ -80,8 +75,7 @@ struct Sim {
     std::lock_guard<std::mutex> g(mu);
     unfenced[tid] = 0;
   }
-  static void sync() { warp_meet[tid / 32](true); }
-  static bool all(bool ok) { return warp_meet[tid / 32](ok); }
+  static void sync() { warp_meet[tid / 32](); }
 };
 
 // the copy engine: chunks land a little after they were issued
@@ -142,10 +136,9 @@ int run(int nch, int which) {
           cs.init();
           cs.begin(nch, issue);
         }
-        cta_meet(true);
+        cta_meet();
         for (int c = 0; c < nch; ++c) {
-          if (!cs.wait(c)) break;
-          {
+          if (cs.wait(c)) {
             std::lock_guard<std::mutex> g(mu);
             wrong += stage[c % STAGES] != c;
             unfenced[tid] |= 1u << (c % STAGES);
@@ -157,7 +150,7 @@ int run(int nch, int which) {
           std::lock_guard<std::mutex> g(mu);
           fail = 1;
         }
-        cta_meet(true);
+        cta_meet();
         if (fail && tid == 0) err = cs.drain();
         if (tid == 0) {
           std::lock_guard<std::mutex> g(mu);
