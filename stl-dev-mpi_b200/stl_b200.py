@@ -955,10 +955,12 @@ class PatchEngine:
         (which gathers them while it copies them)."""
         if len(maps) != len(self.ids):
             raise ValueError(f"{len(maps)} patches given for {len(self.ids)} selected discs")
-        flat = [np.ascontiguousarray(m, dtype=np.float64) for m in maps]
-        for i, (m, size) in enumerate(zip(flat, self._sizes)):
-            if m.shape != (size,):
+        flat = []
+        for i, (m, size) in enumerate(zip(maps, self._sizes)):
+            m = np.asarray(m, dtype=np.float64)
+            if m.shape != (size,):  # before ascontiguousarray, which makes a scalar a vector
                 raise ValueError(f"patch {i} has shape {m.shape}; its disc holds {size} pixels")
+            flat.append(np.ascontiguousarray(m))
         return flat, (_VOID * len(flat))(*[m.ctypes.data for m in flat])
 
     def forward(self, maps, centres=None, radius=None, core=None, moments=True, generation=0, out=None):
