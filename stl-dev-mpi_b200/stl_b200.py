@@ -985,6 +985,10 @@ class PatchEngine:
                         and out.shape == (b, self.ncoeff)):
                     raise ValueError(f"out must be a C-contiguous complex128 array of shape {(b, self.ncoeff)}")
                 values = out
+                # the library reads the patches of a later group of discs after it wrote
+                # the statistics of an earlier one
+                if any(np.may_share_memory(out, m) for m in flat):
+                    flat, parts = self._parts([m.copy() for m in flat])
             variance = np.empty((b, self.ncoeff if moments else 0), dtype=np.float64)
             self._generation = None
             self._dense = isinstance(maps, np.ndarray)

@@ -37,3 +37,21 @@ def test_parts_equal_the_packed_patches(nside, radii):
     with pytest.raises(ValueError):
         pe.forward([x[:-1] for x in patches], moments=False)
     pe.close()
+
+
+def test_statistics_may_overwrite_the_patches():
+    """``out`` in the patches' own memory: the discs of a later engine group are read
+    after the statistics of an earlier one were written."""
+    import stl_b200
+    rng = np.random.default_rng(5)
+    pe = stl_b200.PatchEngine(32, 2, autotune=False, group_pixels=1)  # a group a disc
+    ids = pe.select(rng.standard_normal((3, 3)), 40.0)
+    assert sum(i.size for i in ids) > 2 * 3 * pe.ncoeff
+    buf = rng.standard_normal(sum(i.size for i in ids))
+    patches = np.split(buf, np.cumsum([i.size for i in ids])[:-1])
+    want = pe.forward([p.copy() for p in patches], moments=False)[0]
+    out = buf[-2 * want.size:].view(np.complex128).reshape(want.shape)  # the last patch among it
+    got = pe.forward(patches, moments=False, out=out)[0]
+    assert got is out
+    np.testing.assert_array_equal(got, want)
+    pe.close()
