@@ -113,6 +113,12 @@ int stlp_prepare(StlpHandle* h);
  * engine.rs:811-818, reported by stlp_info). */
 int stlp_profile(StlpHandle* h, int on, int reset);
 
+/* Device address of the int32 error flag of the handle's sweeps, which the
+ * kernels set when a wait on a staged copy ran out.  A call that finds it nonzero
+ * after its sweep clears it and fails; a gradient array it was given is left as
+ * it was.  (No reference counterpart.) */
+int stlp_error_flag(StlpHandle* h, uint64_t* out);
+
 /* Copy of the current forward state (the loaded maps; the fields are
  * recomputed by stlp_restore); NULL on failure.  (lib.rs:647-659) */
 StlpSnapshot* stlp_checkpoint(StlpHandle* h);

@@ -191,6 +191,16 @@ int stlp_prepare(StlpHandle* h) {
   });
 }
 
+int stlp_error_flag(StlpHandle* h, uint64_t* out) {
+  return guard<int>(-1, [&] {
+    require(h != nullptr && out != nullptr, "null argument");
+    h->activate();
+    h->engine->prepare();
+    *out = reinterpret_cast<uint64_t>(h->engine->error_flag());
+    return 0;
+  });
+}
+
 int stlp_profile(StlpHandle* h, int on, int reset) {
   return guard<int>(-1, [&] {
     require(h != nullptr, "null handle");

@@ -217,12 +217,16 @@ class HostStage {
       });
     });
   }
-  // host dst <- device src (n bytes) after the work queued on s; synchronises
-  void to_host(void* dst, const void* src, size_t n, cudaStream_t s) {
+  // host dst <- device src (n bytes) after the work queued on s; synchronises.
+  // arrived() is called once the work before the copy is done, before dst is
+  // written (it may throw)
+  template <typename F>
+  void to_host(void* dst, const void* src, size_t n, cudaStream_t s, F&& arrived) {
     if (n < kDirect) {  // through a small pinned buffer
       void* p = small(n);
       STL_CUDA(cudaMemcpyAsync(p, src, n, cudaMemcpyDeviceToHost, s));
       STL_CUDA(cudaStreamSynchronize(s));
+      arrived();
       host_copy(dst, p, n, false);
       return;
     }
@@ -231,6 +235,7 @@ class HostStage {
     auto drain = [&](size_t c) {  // chunk c: from its pinned buffer to dst
       const size_t off = c * kChunk, len = std::min(kChunk, n - off);
       STL_CUDA(cudaEventSynchronize(ev_[c & 1]));
+      if (c == 0) arrived();
       CopyPool::get().copy(static_cast<char*>(dst) + off, buf_[c & 1].p, len);
     };
     for (size_t c = 0; c < nc; ++c) {
@@ -243,12 +248,14 @@ class HostStage {
   }
   // host doubles dst <- device floats src (n floats), widened on the host: half
   // the bytes cross PCIe; synchronises
-  void to_host_widen(double* dst, const float* src, size_t n, cudaStream_t s) {
+  template <typename F>
+  void to_host_widen(double* dst, const float* src, size_t n, cudaStream_t s, F&& arrived) {
     const size_t bytes = n * sizeof(float);
     if (bytes < kDirect) {
       float* p = static_cast<float*>(small(bytes));
       STL_CUDA(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, s));
       STL_CUDA(cudaStreamSynchronize(s));
+      arrived();
       host_widen(dst, p, n);
       return;
     }
@@ -257,6 +264,7 @@ class HostStage {
     auto drain = [&](size_t c) {
       const size_t off = c * kChunk, len = std::min(kChunk, bytes - off);
       STL_CUDA(cudaEventSynchronize(ev_[c & 1]));
+      if (c == 0) arrived();
       CopyPool::get().copy(reinterpret_cast<char*>(dst) + 2 * off, buf_[c & 1].p, len, false, true);
     };
     for (size_t c = 0; c < nc; ++c) {
@@ -1098,16 +1106,23 @@ class EngineImpl final : public Engine {
   }
 
   // reverse_impl queues the sweep and the copy of its error flag; the caller
-  // waits for the stream and then checks the flag (finish_reverse)
+  // waits for the stream and then checks the flag (finish_reverse).  The
+  // gradient of a failed sweep does not reach out: the host copies check the flag
+  // before they write it, the device one reads it in the kernel that writes.
   void reverse_host(const double* cot, double* out) override {
     const auto t0 = std::chrono::steady_clock::now();
     reverse_impl(cot);
     i64 n = (i64)opt_.B * npix(0);
+    auto arrived = [&] {
+      if (!*err_pin_.as<int>()) return;
+      STL_CUDA(cudaStreamSynchronize(stream_));  // the chunks still in flight
+      finish_reverse(t0);                        // throws
+    };
     if (!hi(0)) {  // FP32 gradients: moved as floats and widened on the host (exact)
       prof_.launch(Profiler::ELEM, 1, n * (4.0 + esz(0)), 0.0, stream_, [&] {
         to_map_major<float, float>(gX_[0].as<float>(), in_f64_.as<float>(), npix(0), opt_.B, stream_);
       });
-      io_.to_host_widen(out, in_f64_.as<float>(), (size_t)n, stream_);
+      io_.to_host_widen(out, in_f64_.as<float>(), (size_t)n, stream_, arrived);
       finish_reverse(t0);
       return;
     }
@@ -1117,7 +1132,7 @@ class EngineImpl final : public Engine {
         to_map_major<U, double>(gX_[0].as<U>(), in_f64_.as<double>(), npix(0), opt_.B, stream_);
       });
     });
-    io_.to_host(out, in_f64_.p, n * 8, stream_);
+    io_.to_host(out, in_f64_.p, n * 8, stream_, arrived);
     finish_reverse(t0);
   }
 
@@ -1125,11 +1140,12 @@ class EngineImpl final : public Engine {
     const auto t0 = std::chrono::steady_clock::now();
     reverse_impl(cot);
     i64 n = (i64)opt_.B * npix(0);
+    const int* err = err_.as<int>();
     prof_.launch(Profiler::ELEM, 1, n * ((f32 ? 4.0 : 8.0) + esz(0)), 0.0, stream_, [&] {
       typed(0, [&](auto t) {
         using U = typename decltype(t)::type;
-        if (f32) to_map_major<U, float>(gX_[0].as<U>(), static_cast<float*>(out), npix(0), opt_.B, stream_);
-        else to_map_major<U, double>(gX_[0].as<U>(), static_cast<double*>(out), npix(0), opt_.B, stream_);
+        if (f32) to_map_major<U, float>(gX_[0].as<U>(), static_cast<float*>(out), npix(0), opt_.B, stream_, nullptr, err);
+        else to_map_major<U, double>(gX_[0].as<U>(), static_cast<double*>(out), npix(0), opt_.B, stream_, nullptr, err);
       });
     });
     STL_CUDA(cudaStreamSynchronize(stream_));
@@ -1139,7 +1155,7 @@ class EngineImpl final : public Engine {
   size_t host_to_device(void* dst, const void* src, size_t n, bool check) override {
     return io_.to_device(dst, src, n, stream_, check);
   }
-  void device_to_host(void* dst, const void* src, size_t n) override { io_.to_host(dst, src, n, stream_); }
+  void device_to_host(void* dst, const void* src, size_t n) override { io_.to_host(dst, src, n, stream_, [] {}); }
 
   void reverse_levels(const double* cot, double* const* out) override {
     if (!levels_given_) throw std::runtime_error("per-level cotangents need maps given at every level");

@@ -455,7 +455,9 @@ void to_pixel_major(const Tin* in, Tout* out, i64 N, int B, cudaStream_t s, cons
 // FP64 values as FP32 pairs (hi rounded, lo the rounded rest) and back
 void split_f64(const double* x, float* hi, float* lo, i64 n, cudaStream_t s);
 void join_f64(const float* hi, const float* lo, double* x, i64 n, cudaStream_t s);
+// failed (device, or null): out is left as it is when *failed != 0
 template <typename Tin, typename Tout>
-void to_map_major(const Tin* in, Tout* out, i64 N, int B, cudaStream_t s, const double* add = nullptr);
+void to_map_major(const Tin* in, Tout* out, i64 N, int B, cudaStream_t s, const double* add = nullptr,
+                  const int* failed = nullptr);
 
 }  // namespace stl

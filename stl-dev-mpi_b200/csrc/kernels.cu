@@ -2701,7 +2701,8 @@ __global__ void k_join_f64(const float* __restrict__ hi, const float* __restrict
 }
 template <typename Tin, typename Tout, typename I>
 __global__ void k_to_map_major(const Tin* __restrict__ in, Tout* __restrict__ out, i64 N, int B,
-                               const double* __restrict__ add) {
+                               const double* __restrict__ add, const int* __restrict__ failed) {
+  if (failed && *failed) return;
   const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;  // over B * N, output order
   if ((i64)i >= N * B) return;
   const int b = (int)(i / (I)N);
@@ -4305,9 +4306,11 @@ void join_f64(const float* hi, const float* lo, double* x, i64 n, cudaStream_t s
 }
 
 template <typename Tin, typename Tout>
-void to_map_major(const Tin* in, Tout* out, i64 N, int B, cudaStream_t s, const double* add) {
-  if (N * B < ((i64)1 << 31)) k_to_map_major<Tin, Tout, uint32_t><<<nblocks(N * B, 256), 256, 0, s>>>(in, out, N, B, add);
-  else k_to_map_major<Tin, Tout, i64><<<nblocks(N * B, 256), 256, 0, s>>>(in, out, N, B, add);
+void to_map_major(const Tin* in, Tout* out, i64 N, int B, cudaStream_t s, const double* add, const int* failed) {
+  if (N * B < ((i64)1 << 31))
+    k_to_map_major<Tin, Tout, uint32_t><<<nblocks(N * B, 256), 256, 0, s>>>(in, out, N, B, add, failed);
+  else
+    k_to_map_major<Tin, Tout, i64><<<nblocks(N * B, 256), 256, 0, s>>>(in, out, N, B, add, failed);
   STL_CUDA(cudaGetLastError());
 }
 
@@ -4349,9 +4352,9 @@ template void to_pixel_major<double, float>(const double*, float*, i64, int, cud
 template void to_pixel_major<double, double>(const double*, double*, i64, int, cudaStream_t, const double*, double*);
 template void to_pixel_major<float, float>(const float*, float*, i64, int, cudaStream_t, const double*, float*);
 template void to_pixel_major<float, double>(const float*, double*, i64, int, cudaStream_t, const double*, double*);
-template void to_map_major<float, double>(const float*, double*, i64, int, cudaStream_t, const double*);
-template void to_map_major<double, double>(const double*, double*, i64, int, cudaStream_t, const double*);
-template void to_map_major<float, float>(const float*, float*, i64, int, cudaStream_t, const double*);
-template void to_map_major<double, float>(const double*, float*, i64, int, cudaStream_t, const double*);
+template void to_map_major<float, double>(const float*, double*, i64, int, cudaStream_t, const double*, const int*);
+template void to_map_major<double, double>(const double*, double*, i64, int, cudaStream_t, const double*, const int*);
+template void to_map_major<float, float>(const float*, float*, i64, int, cudaStream_t, const double*, const int*);
+template void to_map_major<double, float>(const double*, float*, i64, int, cudaStream_t, const double*, const int*);
 
 }  // namespace stl

@@ -62,6 +62,7 @@ def lib():
             "stlp_prepare": ([_VOID], C.c_int),
             "stlp_set_stream": ([_VOID, u64], C.c_int),
             "stlp_profile": ([_VOID, C.c_int, C.c_int], C.c_int),
+            "stlp_error_flag": ([_VOID, C.POINTER(u64)], C.c_int),
             "stlp_set_masks": ([_VOID, _D, sz], C.c_int),
             "stlp_synthesize_device": ([_VOID, u64, sz, _D, sz, _D, C.c_char_p, _D, sz], C.c_int64),
             "stlp_native_pixels": ([_VOID, _SIZE], C.c_int),
