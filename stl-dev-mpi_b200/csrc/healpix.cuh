@@ -288,24 +288,34 @@ HD void rotation_matrix(double theta, double phi, int g, int G, int gauge, doubl
       out[3 * i + j] = rg[3 * i] * base[j] + rg[3 * i + 1] * base[3 + j] + rg[3 * i + 2] * base[6 + j];
 }
 
-// pixel at the extended coordinates (ex, ey) of `face` (dia.rs:46-77);
-// false in the quadrant missing at a vertex of three faces
-HD bool ext_pix(i64 face, i64 ex, i64 ey, i64 nside, int order, i64& out) {
+// the face on side nb (0 .. 8, row by row, 4 the face itself) of `face`, or -1
+// (vertices of three faces), and how its frame is flipped: bit 0 x, bit 1 y, bit 2
+// x and y exchanged
+HD int neighbour_face(int nb, i64 face) {
   const signed char NB_FACE[9][12] = {
       {8, 9, 10, 11, -1, -1, -1, -1, 10, 11, 8, 9}, {5, 6, 7, 4, 8, 9, 10, 11, 9, 10, 11, 8},
       {-1, -1, -1, -1, 5, 6, 7, 4, -1, -1, -1, -1}, {4, 5, 6, 7, 11, 8, 9, 10, 11, 8, 9, 10},
       {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11},       {1, 2, 3, 0, 0, 1, 2, 3, 5, 6, 7, 4},
       {-1, -1, -1, -1, 7, 4, 5, 6, -1, -1, -1, -1}, {3, 0, 1, 2, 3, 0, 1, 2, 4, 5, 6, 7},
       {2, 3, 0, 1, -1, -1, -1, -1, 0, 1, 2, 3}};
+  return NB_FACE[nb][face];
+}
+HD int neighbour_swap(int nb, i64 face) {
   const unsigned char NB_SWAP[9][3] = {{0, 0, 3}, {0, 0, 6}, {0, 0, 0}, {0, 0, 5}, {0, 0, 0},
                                        {5, 0, 0}, {0, 0, 0}, {6, 0, 0}, {3, 0, 0}};
+  return NB_SWAP[nb][face >> 2];
+}
+
+// pixel at the extended coordinates (ex, ey) of `face` (dia.rs:46-77);
+// false in the quadrant missing at a vertex of three faces
+HD bool ext_pix(i64 face, i64 ex, i64 ey, i64 nside, int order, i64& out) {
   i64 x = ex, y = ey;
   int nb = 4;
   if (x < 0) { x += nside; nb -= 1; } else if (x >= nside) { x -= nside; nb += 1; }
   if (y < 0) { y += nside; nb -= 3; } else if (y >= nside) { y -= nside; nb += 3; }
-  int f = NB_FACE[nb][face];
+  int f = neighbour_face(nb, face);
   if (f < 0) return false;
-  int bits = NB_SWAP[nb][face >> 2];
+  int bits = neighbour_swap(nb, face);
   if (bits & 1) x = nside - x - 1;
   if (bits & 2) y = nside - y - 1;
   if (bits & 4) { i64 t = x; x = y; y = t; }
@@ -317,20 +327,12 @@ HD bool ext_pix(i64 face, i64 ex, i64 ey, i64 nside, int order, i64& out) {
 // pixel (x, y) of `face` are the cell (the inverse of ext_pix near a pixel);
 // false when the cell is not that near
 HD bool rel_cell(i64 face, i64 x, i64 y, i64 cell, i64 nside, int order, int reach, int& dx, int& dy) {
-  const signed char NB_FACE[9][12] = {
-      {8, 9, 10, 11, -1, -1, -1, -1, 10, 11, 8, 9}, {5, 6, 7, 4, 8, 9, 10, 11, 9, 10, 11, 8},
-      {-1, -1, -1, -1, 5, 6, 7, 4, -1, -1, -1, -1}, {4, 5, 6, 7, 11, 8, 9, 10, 11, 8, 9, 10},
-      {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11},       {1, 2, 3, 0, 0, 1, 2, 3, 5, 6, 7, 4},
-      {-1, -1, -1, -1, 7, 4, 5, 6, -1, -1, -1, -1}, {3, 0, 1, 2, 3, 0, 1, 2, 4, 5, 6, 7},
-      {2, 3, 0, 1, -1, -1, -1, -1, 0, 1, 2, 3}};
-  const unsigned char NB_SWAP[9][3] = {{0, 0, 3}, {0, 0, 6}, {0, 0, 0}, {0, 0, 5}, {0, 0, 0},
-                                       {5, 0, 0}, {0, 0, 0}, {6, 0, 0}, {3, 0, 0}};
   i64 cx, cy, cf;
   nest2xyf(cell, order, cx, cy, cf);
   for (int nb = 0; nb < 9; ++nb) {
-    if (NB_FACE[nb][face] != cf) continue;
+    if (neighbour_face(nb, face) != cf) continue;
     i64 a = cx, b = cy;
-    const int bits = NB_SWAP[nb][face >> 2];
+    const int bits = neighbour_swap(nb, face);
     if (bits & 4) { i64 t = a; a = b; b = t; }
     if (bits & 2) b = nside - b - 1;
     if (bits & 1) a = nside - a - 1;

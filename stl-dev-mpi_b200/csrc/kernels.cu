@@ -3777,7 +3777,7 @@ __global__ void __launch_bounds__(kCrossThreads) k_cross_rev(i64 N, int K, int B
 // level 2 (K = 13; levels 0 and 1 run in registers): the deeper levels have too
 // few pixel ranges to fill the GPU with a quarter of the CTAs (measured slower at
 // K = 17, 21)
-constexpr int kCross4MaxK = 13;
+constexpr int kCross4K = 13, kCross4Ent = 4;  // 4 (K^2 + 1) = 680 entries: 3 of 256 a thread
 
 template <typename T>
 __device__ __forceinline__ void load_gauges(const typename V2<T>::type* src, double2 v[4]) {
@@ -4135,25 +4135,16 @@ void launch_cross_fwd(unsigned grid, size_t smem, cudaStream_t s, i64 N, int K, 
 template <typename T, bool MOM>
 void launch_cross_fwd(int nent, unsigned grid, size_t smem, cudaStream_t s, i64 N, int K, int Bm, const T* z,
                       const T* br, const uint8_t* mask, i64 chunk, int PC, double* partials) {
-  if (nent <= 1) launch_cross_fwd<T, MOM, 1>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
-  else if (nent <= 2) launch_cross_fwd<T, MOM, 2>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
+  if (nent <= 2) launch_cross_fwd<T, MOM, 2>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
   else if (nent <= 4) launch_cross_fwd<T, MOM, 4>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
   else launch_cross_fwd<T, MOM, kCrossMaxEnt>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
 }
 
-template <typename T, bool MOM, int NENT>
-void launch_cross_fwd4(unsigned grid, size_t smem, cudaStream_t s, i64 N, int K, int Bm, const T* z, const T* br,
-                       const uint8_t* mask, i64 chunk, int PC, double* partials) {
-  if (smem > 48 * 1024) allow_dynamic_smem(k_cross_fwd4<T, MOM, NENT>);
-  k_cross_fwd4<T, MOM, NENT><<<grid, kCrossThreads, smem, s>>>(N, K, Bm, z, br, mask, chunk, PC, partials);
-}
 template <typename T, bool MOM>
-void launch_cross_fwd4(int nent, unsigned grid, size_t smem, cudaStream_t s, i64 N, int K, int Bm, const T* z,
-                       const T* br, const uint8_t* mask, i64 chunk, int PC, double* partials) {
-  if (nent <= 1) launch_cross_fwd4<T, MOM, 1>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
-  else if (nent <= 2) launch_cross_fwd4<T, MOM, 2>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
-  else if (nent <= 4) launch_cross_fwd4<T, MOM, 4>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
-  else launch_cross_fwd4<T, MOM, kCrossMaxEnt>(grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
+void launch_cross_fwd4(unsigned grid, size_t smem, cudaStream_t s, i64 N, int Bm, const T* z, const T* br,
+                       const uint8_t* mask, i64 chunk, int PC, double* partials) {
+  if (smem > 48 * 1024) allow_dynamic_smem(k_cross_fwd4<T, MOM, kCross4Ent>);
+  k_cross_fwd4<T, MOM, kCross4Ent><<<grid, kCrossThreads, smem, s>>>(N, kCross4K, Bm, z, br, mask, chunk, PC, partials);
 }
 
 template <typename T>
@@ -4174,18 +4165,17 @@ void cross_forward(int K, i64 N, int Bm, const T* z, const T* br, const uint8_t*
     STL_CUDA(cudaGetLastError());
     return;
   }
-  if (K <= kCross4MaxK) {  // the four gauges a CTA
+  if (K == kCross4K) {  // the four gauges a CTA
     const int E4 = 4 * (K * K + 1), NE = std::min(E4, kCrossThreads), Q = kCrossThreads / NE;
-    const int nent = (E4 + NE - 1) / NE;
     const int per = 4 * 2 * (K + 1) * (moments ? 24 : 16);
     const int PC = std::max(8, std::min(256, (48 * 1024) / per));
-    const size_t smem = std::max((size_t)PC * per, sizeof(double) * (size_t)Q * NE * kCrossMaxEnt * 3);
+    const size_t smem = std::max((size_t)PC * per, sizeof(double) * (size_t)Q * NE * kCross4Ent * 3);
     const i64 chunk = (N + nblk - 1) / nblk;
     const unsigned grid = (unsigned)nblk * (unsigned)(Bm / 2);
     if (moments)
-      launch_cross_fwd4<T, true>(nent, grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
+      launch_cross_fwd4<T, true>(grid, smem, s, N, Bm, z, br, mask, chunk, PC, partials);
     else
-      launch_cross_fwd4<T, false>(nent, grid, smem, s, N, K, Bm, z, br, mask, chunk, PC, partials);
+      launch_cross_fwd4<T, false>(grid, smem, s, N, Bm, z, br, mask, chunk, PC, partials);
     STL_CUDA(cudaGetLastError());
     const i64 rows = (i64)Bm / 2 * 4, total = rows * cross_slots(K);
     k_reduce_partials<<<(unsigned)std::min<i64>((total + 31) / 32, 4096), 256, 0, s>>>(partials, nblk, (int)rows,
@@ -4196,7 +4186,7 @@ void cross_forward(int K, i64 N, int Bm, const T* z, const T* br, const uint8_t*
   const int E = K * K + 1, NE = std::min(E, kCrossThreads), Q = kCrossThreads / NE;
   const int nent = (E + NE - 1) / NE;
   if (nent > kCrossMaxEnt) throw std::runtime_error("too many cross terms per level");
-  const int NENT = nent <= 1 ? 1 : nent <= 2 ? 2 : nent <= 4 ? 4 : kCrossMaxEnt;
+  const int NENT = nent <= 2 ? 2 : nent <= 4 ? 4 : kCrossMaxEnt;  // K >= 17: two at least
   const int PC = cross_chunk(K, moments);
   const size_t stage = (sizeof(double2) + (moments ? sizeof(double) : 0)) * (size_t)PC * 2 * (K + 1);
   const size_t smem = std::max(stage, sizeof(double) * (size_t)Q * NE * NENT * 3);
