@@ -1323,13 +1323,13 @@ class EngineImpl final : public Engine {
 
  private:
   // Algorithmic traffic of one wavelet launch over R rows: the used
-  // coefficients of the stored rows (2L values and a 4-byte cell index per
-  // cell read; a quarter of the rows on the full sky), the input rows read
+  // coefficients of the stored rows (2L values and, but for the grid layout, a
+  // 4-byte cell index per cell read; a quarter of the rows on the full sky), the input rows read
   // once, the complex outputs written once (plus |z|, or the
   // read-modify-write of an accumulated adjoint).
   double conv_bytes(const ConvOp& op, int R, bool fwd, bool extra) const {
     const double s = op.dtype == DType::F64 ? 8.0 : 4.0, N = (double)op.n_rows, D = op.mean_slots;
-    double coef = (double)op.n_rep * D * (8.0 * s + 4.0);
+    double coef = (double)op.n_rep * D * (8.0 * s + (op.grid ? 0.0 : 4.0));
     double field = fwd ? R * N * s + R * N * 8.0 * s : R * N * 8.0 * s + R * N * s;
     if (extra) field += fwd ? R * N * 4.0 * s : R * N * s;
     return coef + field;
@@ -1541,8 +1541,8 @@ class EngineImpl final : public Engine {
                    conv_adjoint<U>(op, gBr_.as<U>(), R, gmod, true, s, adj_ptr(), err_.as<int>(), nullptr,
                                    tile(n, T_ADJ_BR));
                  });
-    // the modulus VJP of z (gZ += gmod z / |z|): inside the coloured adjoint
-    // of z when the operator has it, else its own pass
+    // the modulus VJP of z (gZ += gmod z / |z|): inside the adjoint of z where
+    // its kernel takes it (grid, coloured, tensor cores), else its own pass
     ModulusAdd<U> madd;
     madd.z = zf<U>(n);
     madd.g = gmod + n * L;

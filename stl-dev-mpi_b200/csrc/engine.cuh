@@ -100,9 +100,9 @@ inline size_t dsize(DType t) { return t == DType::F64 ? 8 : 4; }
 // Geometry of one wavelet operator: output rows reading an input grid.
 struct ConvSpec {
   i64 nside = 0;
-  // FP32 full sky: 0 the coloured layout only (CUDA cores), 1 the tensor-core
-  // layout for the forward and the coloured one for the adjoint, 2 the
-  // tensor-core layout for both
+  // FP32 full sky: 0 the CUDA-core layouts only (grid, coloured below nside 16),
+  // 1 the tensor-core layout for the forward and the coloured one for the
+  // adjoint, 2 the tensor-core layout for both
   int tensor_cores = 0;
   int ksz = 5, G = 4, gauge = 0;
   double eps = 0.0;
@@ -168,9 +168,9 @@ struct ConvOp {
   // the face frame, the same for all its rows, so the cells of a slot are the
   // tile's block moved by it: no index per row, no two rows on one cell, and
   // regular shared-memory addresses.  The displacements of the rows of a tile
-  // differ little (128 rows at nside 1024: 45.6 of them a tile for 44.4 cells a
-  // row; 64: 53.6 for 44.1; 16: 66.3 for 44.0), so the slots hold no more padding
-  // than a colouring of the tile's entries (48 slots) does.
+  // differ little: 44 cells a row, and with the padding to kGridPad 46.5 slots a
+  // tile at nside 1024 and more, 48.3 at 256, 52.0 at 64, 64.0 at 16 (48 for a
+  // colouring of the tile's entries: less only at the coarse levels).
   bool grid = false;
   DevMem g_start;            // int64 [n_tiles + 1]: first slot of every tile (a multiple of kGridPad)
   DevMem g_off;              // int32 [slots]: dy kGridP + dx
@@ -179,7 +179,7 @@ struct ConvOp {
   DevMem g_lpos;             // uint16 [n_tiles][ncs]: grid position of every tile cell
   int G = 4;
   double mean_slots = 0.0;   // cells read per row, averaged over the rows
-  // Tensor-core layout (FP32 full sky; replaces the coloured one).  Tiles of
+  // Tensor-core layout (FP32 full sky, on request; replaces the grid one).  Tiles of
   // kMmaRows stored rows; per tile a plane of input cells in which cell c
   // sits at 4 (its rank among the tile's cells of its class) + class, the
   // class being c's NESTED bits x0 + 2 y0 (the parity of its face
@@ -205,8 +205,8 @@ struct ConvOp {
   size_t bytes() const {
     return cell.bytes + coef.bytes + tent.bytes + coefT.bytes + rowsum.bytes + tile_cells.bytes + tile_ncells.bytes +
            tile_slots.bytes + lcell.bytes + lcell_t.bytes + tile_ent.bytes + tile_off.bytes + coff.bytes +
-           clist.bytes + g_start.bytes + g_off.bytes + g_coef.bytes + g_pos.bytes + g_lpos.bytes + m_coef.bytes + m_cells.bytes + m_lc.bytes + m_wlc.bytes + m_winv.bytes + m_rowch.bytes +
-           m_tch.bytes;
+           clist.bytes + g_start.bytes + g_off.bytes + g_coef.bytes + g_pos.bytes + g_lpos.bytes + m_coef.bytes +
+           m_cells.bytes + m_lc.bytes + m_wlc.bytes + m_winv.bytes + m_rowch.bytes + m_tch.bytes;
   }
 };
 constexpr int kMmaRows = 64;      // stored rows per tile of the tensor-core layout
@@ -292,10 +292,10 @@ template <typename T>
 void conv_forward(const ConvOp& op, const T* x, int R, T* out, T* mod, int mod_pix, int mod_row, int mod_off,
                   cudaStream_t s, int* err = nullptr, const double* rc = nullptr, int rb = 0);
 std::vector<int> conv_forward_choices(const ConvOp& op, size_t elem, int R, bool err);
-//  With scratch, operators in the coloured layout use the coloured adjoint
-//  (bounded waits on its bulk copies set *err on timeout), other operators
-//  with tile tables the two-phase adjoint; otherwise the transposed gather.
-//  madd (coloured adjoint only): first add the modulus VJP to the input,
+//  With scratch, operators in the grid, coloured and tensor-core layouts use the
+//  adjoint of their layout (bounded waits on its bulk copies set *err on
+//  timeout), other operators with tile tables the two-phase adjoint; otherwise
+//  the transposed gather.  madd (where conv_adjoint_fuses_modulus): first add the modulus VJP to the input,
 //  gy[p][r][l] += g[p g_pix + r g_row + l] z[p][r][l] / |z[p][r][l]| (0 at
 //  z = 0), the rows r being the maps.
 template <typename T>

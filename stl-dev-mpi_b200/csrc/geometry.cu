@@ -1328,8 +1328,8 @@ static void build_conv_t(const ConvSpec& sp, const std::vector<double>& kernel, 
   const i64 n_cells = sym ? a.n_in / 4 : a.n_in;  // stored cells == stored rows on the full sky
   if (sym && n_cells != a.n_rows) throw std::runtime_error("symmetric operator needs rows == cells");
   if (!sym && n_cells != a.n_rows) throw std::runtime_error("rows and grid must coincide");
-  // row-centric adjoint tiles (full sky): the distinct cells of every tile
-  // of kAdjTile stored rows, then the edge colouring of its entries
+  // tiles of stored rows (full sky): the distinct cells of every tile, then the
+  // grid layout (nside 16 and more) or the edge colouring of its entries
   op.adj_tiles = false;
   op.colored = false;
   op.grid = false;

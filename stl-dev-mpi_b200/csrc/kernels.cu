@@ -399,7 +399,10 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const int32_t* __restrict__ ce
 // share each coefficient read.  The CTA gathers the tile's cells (4
 // rotations x RB values) into shared memory once; the coefficients and
 // tile-cell indices of the tile stream through shared memory in chunks of
-// SC slots, two stages deep, by bulk asynchronous copies.
+// SC slots, two stages deep, by bulk asynchronous copies.  For full-sky levels below
+// nside 16 (FP64), and for a level whose tiles the grid layout cannot hold (none at
+// nside 16 to 1024 with either kernel size): the FP32 instances are there for that
+// fallback of the builder only.
 constexpr int kFwdThreads = 4 * kAdjTile;
 // cells of a gather plane: at least nc + 1, plane bytes = 32 mod 128 when
 // reachable (within 32 extra cells)

@@ -43,8 +43,8 @@ struct Options {
   int device = 0;
   bool autotune = true;  // time the tile heights of the wavelet and decimation launches at prepare
   // FP32 full-sky wavelets on the tensor cores (3xTF32 mma.sync): 0 none
-  // (the CUDA-core kernels of the coloured layout, the default: as fast,
-  // a single layout, closer to FP64), 1 the forward (the adjoint on the
+  // (the CUDA-core kernels, the default: faster in the grid layout, a single
+  // layout, closer to FP64), 1 the forward (the adjoint on the
   // CUDA cores), 2 forward and adjoint
   int tensor_cores = 0;
   // Two channels and the plan of their cross terms only (c1 != c2: S1 of the
