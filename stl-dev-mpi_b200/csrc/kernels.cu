@@ -92,10 +92,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned phase) {
   }
   return false;
 }
-// Between a thread's reads of a stage of shared memory and the barrier after which
-// the copy engine (the async proxy) writes the stage again: without the fence the
-// barrier does not order the two.
-__device__ __forceinline__ void stage_reads_done() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Between the barrier after the reads of a stage of shared memory and the copy that
+// writes it again, by the thread that issues the copy: the copy engine is another
+// proxy (async), and without the fence the barrier does not order the two.
+__device__ __forceinline__ void refill_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // the stage protocol's barriers (StageStream)
 struct StageBarriers {
   static __device__ __forceinline__ void init(uint64_t* bar, unsigned count) { mbar_init(bar, count); }
@@ -105,7 +105,7 @@ struct StageBarriers {
   }
   static __device__ __forceinline__ bool wait(uint64_t* bar, unsigned phase) { return mbar_wait(bar, phase); }
   static __device__ __forceinline__ void arrive(uint64_t* bar) { mbar_arrive(bar); }
-  static __device__ __forceinline__ void reads_done() { stage_reads_done(); }
+  static __device__ __forceinline__ void refill_fence() { stl::refill_fence(); }
   static __device__ __forceinline__ void sync() { __syncwarp(); }
 };
 
@@ -883,11 +883,12 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
         dot8_rows<RB>(w, g, a);
         addR_shared<RB>(acc + ((size_t)lc * 4 + k) * RB, a);
       }
-      if (sl + 1 < sn) __syncthreads();  // the slot's sums are in: the next slot may read them
+      __syncthreads();  // the slot's sums are in: the next slot may read them
     }
-    stage_reads_done();
-    __syncthreads();
-    if (tid == 0 && c + 2 < nch) issue(c + 2);
+    if (tid == 0 && c + 2 < nch) {
+      refill_fence();
+      issue(c + 2);
+    }
   }
   if (fail) {
     bool drained = true;
@@ -916,8 +917,7 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
 // coefficients: they arrive once a CTA by bulk copies, in stages of grid_sc()
 // slots.  Measured on one B200 (nside 1024, J 9, B 4, FP32, a forward and its
 // VJP): forward 14.5 -> 9.6 ms, adjoint 21.4 -> 15.6 ms; FP64, nside 512, J 8, B 1: 2.80 ->
-// 2.05 and 5.02 -> 2.82 ms (0.05-0.15 and 0.01-0.06 ms of these are the readers' proxy
-// fences).  The level-0 branch forward at nside 512 keeps the FMA
+// 2.03 and 5.02 -> 2.76 ms.  The level-0 branch forward at nside 512 keeps the FMA
 // pipe 57 % busy (36 % before) with three CTAs an SM of 168 registers a thread; two
 // CTAs (no spills, 255 registers) took 11 % longer.  What bounds it now is the FMA
 // pipe inside the slot loop (about 170 of 160 cycles a slot and scheduler) and
@@ -1630,9 +1630,11 @@ __global__ void __launch_bounds__(kMmaFwdThreads, 2) k_conv_fwd_mma(
         for (int q = 0; q < 4; ++q) acc[i][mt][q] += d[q];
       }
     }
-    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
-    if (tid == 0 && c + NS < nch) issue(c + NS);
+    if (tid == 0 && c + NS < nch) {
+      refill_fence();
+      issue(c + NS);
+    }
   }
   if (fail) {
     bool drained = true;
@@ -1792,9 +1794,11 @@ __global__ void __launch_bounds__(kMmaAdjThreads, 2) k_conv_adj_mma(
         *s1 = v1;
       }
     }
-    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
-    if (tid == 0 && c + NS < nch) issue(c + NS);
+    if (tid == 0 && c + NS < nch) {
+      refill_fence();
+      issue(c + NS);
+    }
   }
   if (fail) {
     bool drained = true;
@@ -2088,9 +2092,11 @@ __global__ void __launch_bounds__(kProdMaxWarps * 32, 1) k_products(
         f[i] = (T)0;
       }
     }
-    stage_reads_done();
     __syncthreads();  // the stage is read: refill it
-    if (threadIdx.x == 0 && c + kProdStages < nchunks) issue(c + kProdStages);
+    if (threadIdx.x == 0 && c + kProdStages < nchunks) {
+      refill_fence();
+      issue(c + kProdStages);
+    }
   }
   if (fail) {
     // wait (bounded) for the copies still in flight into this CTA's stages

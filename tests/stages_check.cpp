@@ -2,8 +2,8 @@
 // one a lane, with mbarriers and barriers of their own: a wait that runs
 // out, in thread 0's refill or in one lane, must leave no lane waiting for another
 // for good, and every copy issued must have landed at the end; no copy may be
-// issued into a stage that a lane has read without a proxy fence since.  Exits
-// nonzero on a failure.
+// issued into a stage that a lane has read without a proxy fence, after the lane's
+// warp released the stage, since.  Exits nonzero on a failure.
 #include "stages.cuh"
 
 #include <chrono>
@@ -56,7 +56,9 @@ struct Meet {  // a barrier of n threads
 Meet warp_meet[kWarps], cta_meet;
 
 thread_local int tid;
-unsigned unfenced[kLanes];  // the stages a lane has read since its last fence
+// the stages a lane has read with no fence since, and those its warp has released
+unsigned unfenced[kLanes], released[kWarps];
+std::map<uint64_t*, int> stage_of_empty;
 std::function<bool(uint64_t*, unsigned)> runs_out;  // the wait of this thread that is made to fail
 
 struct Sim {
@@ -69,11 +71,12 @@ struct Sim {
   }
   static void arrive(uint64_t* bar) {
     std::lock_guard<std::mutex> g(mu);
+    released[tid / 32] |= 1u << stage_of_empty.at(bar);
     arrive_locked(bars[bar]);
   }
-  static void reads_done() {
+  static void refill_fence() {
     std::lock_guard<std::mutex> g(mu);
-    unfenced[tid] = 0;
+    for (int l = 0; l < kLanes; ++l) unfenced[l] &= ~released[l / 32];
   }
   static void sync() { warp_meet[tid / 32](); }
 };
@@ -105,6 +108,8 @@ int run(int nch, int which) {
   uint64_t bar[2 * STAGES];
   int stage[STAGES], fail = 0, err = 0, hung = 0, wrong = 0, in_flight = 0, unordered = 0;
   for (unsigned& u : unfenced) u = 0;
+  for (unsigned& u : released) u = 0;
+  for (int q = 0; q < STAGES; ++q) stage_of_empty[&bar[STAGES + q]] = q;
   for (int& v : stage) v = -1;
   bars.clear();
   for (Meet& m : warp_meet) m = Meet{32};
@@ -142,6 +147,7 @@ int run(int nch, int which) {
             std::lock_guard<std::mutex> g(mu);
             wrong += stage[c % STAGES] != c;
             unfenced[tid] |= 1u << (c % STAGES);
+            released[tid / 32] &= ~(1u << (c % STAGES));
           }
           Sim::sync();  // the slots of the adjoint
           cs.release(c, tid, issue);

@@ -1,7 +1,7 @@
 """The staged coefficient stream of the tiled wavelets (csrc/stages.cuh) on host
 threads: a bounded wait that runs out leaves no lane of a warp waiting for the
-others, the copies in flight land first, and a stage's reads are fenced before the
-copy engine writes it again (a C++ check compiled here)."""
+others, the copies in flight land first, and a fence orders a stage's reads
+before the copy that writes it again (a C++ check compiled here)."""
 import shutil
 import subprocess
 from pathlib import Path
