@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(kAdjCThreads, 2) k_conv_adj_colored(
 // slots.  Measured on one B200 (nside 1024, J 9, B 4, FP32, a forward and its
 // VJP): forward 14.5 -> 9.6 ms, adjoint 21.4 -> 15.6 ms; FP64, nside 512, J 8, B 1: 2.80 ->
 // 2.03 and 5.02 -> 2.76 ms.  The level-0 branch forward at nside 512 keeps the FMA
-// pipe 57 % busy (36 % before) with three CTAs an SM of 168 registers a thread; two
+// pipe 55 % busy (36 % before) with three CTAs an SM of 168 registers a thread; two
 // CTAs (no spills, 255 registers) took 11 % longer.  What bounds it now is the FMA
 // pipe inside the slot loop (about 170 of 160 cycles a slot and scheduler) and
 // the CTAs' prologues and epilogues (a third of their time, partly hidden).
