@@ -927,12 +927,13 @@ class PatchEngine:
                                                            _ptr(cores), counts_p)
             if status:
                 raise _error()
-            self.ids = [self._disc_pixels(i, int(c)) for i, c in enumerate(counts)]
+            ids = [self._disc_pixels(i, int(c)) for i, c in enumerate(counts)]
             per_level = np.empty((n, self.levels), dtype=np.uintp)
             if self._lib.stlp_patch_core_pixels(self._handle, per_level.ctypes.data_as(_SIZE)):
                 raise _error()
             self.native_pixels = per_level.astype(np.float64)[:, self._native]
-            self._sizes, self._cuts = counts, np.cumsum(counts.astype(np.int64))
+            # together: the library reads one size for each of the ids
+            self.ids, self._sizes, self._cuts = ids, counts, np.cumsum(counts.astype(np.int64))
             self._selection = ident
             return self.ids
 

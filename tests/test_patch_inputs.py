@@ -1,5 +1,7 @@
 """The patches a disc engine is given, checked against its selection (no device
-needed: the selection is set by hand)."""
+needed: the selection is set by hand, or made by a stand-in for the library)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -34,3 +36,30 @@ def test_patches_are_converted_to_contiguous_doubles():
         assert all(m.dtype == np.float64 and m.flags.c_contiguous for m in flat)
         assert [a for a in addresses] == [m.ctypes.data for m in flat]
         np.testing.assert_array_equal(flat[1], [0.0, 1.0, 2.0])
+
+
+def test_a_selection_that_fails_leaves_ids_and_sizes_of_one_selection():
+    class Library:
+        fail = False
+
+        def stlp_patch_select(self, handle, vectors, n, radius, core, counts):
+            for i in range(n):
+                counts[i] = 5
+            return 0
+
+        def stlp_patch_ids(self, handle, i, out):
+            return 0
+
+        def stlp_patch_core_pixels(self, handle, out):
+            return int(self.fail)
+
+    pe = selected([])
+    pe._mutex, pe._handle, pe._lib = threading.RLock(), 1, Library()
+    pe._selection, pe.levels, pe._native, pe.nside = None, 2, np.zeros(3, np.int64), 16
+    pe.close = lambda: None
+    pe.select(np.eye(3)[:2], 10.0)
+    assert len(pe.ids) == pe._sizes.size == pe._cuts.size == 2
+    pe._lib.fail = True
+    with pytest.raises((RuntimeError, ValueError)):
+        pe.select(np.eye(3), 20.0)
+    assert len(pe.ids) == pe._sizes.size == pe._cuts.size == 2 and pe._selection is None
