@@ -21,8 +21,8 @@ using namespace std::chrono_literals;
 namespace {
 
 constexpr int kWarps = 2, kLanes = 32 * kWarps;
-constexpr auto kWait = 150ms;     // a bounded wait on an mbarrier
-constexpr auto kHang = 2000ms;    // lanes that meet later than this never do
+constexpr auto kWait = 600ms;     // a bounded wait on an mbarrier
+constexpr auto kHang = 5000ms;    // lanes that meet later than this never do
 
 struct Left {};  // a lane gave up on a barrier that nobody will complete
 
